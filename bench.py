@@ -140,18 +140,17 @@ class Clocks:
         return out
 
 
-# DRAM bytes (reads + writes, dram__bytes.sum) per inner iteration of k_jcg_ir on the 1M-node
-# basin, from one ncu capture of that kernel (the second step's solve of the same 1,000,000-row
-# system with 6 levels: launch bytes / inner iterations of that launch); scaled here by the timed
-# launches' inner iterations.
-JCG_DRAM_BYTES_PER_INNER_ITER = 23.9e6
-
-
 def _jcg_bytes_per_iter(N, nnz, mode):
-    """Algorithmic bytes of one JCG iteration: matrix values + column indices + row pointers,
-    and seven vector passes (read p, invD, x, r; write x, r, p), s_v = 8 (FP64) or 4 (FP32)."""
-    sv = 8 if mode == "fp64" else 4
-    return nnz * (sv + 4) + 4 * (N + 1) + 7 * N * sv
+    """Algorithmic bytes of one iteration.  FP64 (Jacobi-PCG): matrix values + column indices + row
+    pointers, and seven vector passes (read p, invD, x, r; write x, r, p).  Mixed precision (FP32
+    iterations with the coarse correction): the matrix off its diagonal (value + index), the fine
+    product's vectors (read z, u, D; write w), the update's (read z, w, p, s, d, u, D; write p, s, d, u)
+    and the interpolation's (read u, write z), and per coarse level (N/4, N/16, ... rows of about eight
+    entries) the matrix and four vectors in each direction."""
+    if mode == "fp64":
+        return nnz * 12 + 4 * (N + 1) + 7 * N * 8
+    coarse = sum(N / 4.0 ** k for k in range(1, 5))
+    return (nnz - N) * 8 + (4 + 11 + 2) * N * 4 + coarse * 2 * (8 * 8 + 4 * 4)
 
 
 def run_ours(a):
@@ -278,8 +277,7 @@ def run_ours(a):
         "e2e": r["e2e"],
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
-                     "traffic": (None if JCG_DRAM_BYTES_PER_INNER_ITER is None
-                                 else JCG_DRAM_BYTES_PER_INNER_ITER * it_in), "kernel": "k_jcg_ir",
+                     "traffic": None, "kernel": "k_jcg_mg",
                      "peak_kind": peak_kind, "iters_per_launch": it_in, "bytes_per_launch": bytes_launch},
         "clocks": r["clocks"],
         # per step, issued phase by phase: clock, btrack, elevation BC, side preparation, ghat, assembly,
@@ -377,7 +375,7 @@ def run_ensemble(a, stream, local):
                                   "solve_roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                                                      "frac": ach / peak, "peak_kind": peak_kind,
                                                      "bytes_per_launch": byts,
-                                                     "kernel": "k_jcg_ir" if prec == "fp32_ir" else "k_jcg64"}}
+                                                     "kernel": "k_jcg_mg" if prec == "fp32_ir" else "k_jcg64"}}
         m.close()
         del m
         torch.cuda.empty_cache()

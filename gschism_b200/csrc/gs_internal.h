@@ -26,7 +26,8 @@ constexpr int kMaxBfr = 8;
 constexpr int kMaxDeg = 24;        // max node degree supported by the per-row assembly
 constexpr int kVortexParams = 9;  // x0, y0, heading, speed, vmax, rmax, B, rho_air, enabled
 constexpr int kMassBlocks = 256;    // fixed grid of the tracer mass budget (deterministic sums)
-constexpr int kIrVectors = 9;      // FP32 vectors of the refinement solve: (u, w, s, p) x 2, d
+constexpr int kIrVectors = 9;      // FP32 vectors of the stand-alone refinement solve: (u, w, s, p) x 2, d
+constexpr int kMgVectors = 6;      // and of a context's: u, z, w, p, s, d
 
 // Device error bits (gs_stats.error_flags)
 enum : int {
@@ -58,9 +59,9 @@ enum : int {
 };
 struct LaunchShape { int block, per_sm; };
 struct JcgTiling {
-    int tiles = 592;        // tiles of a large member (one per block of a 4-blocks-per-SM grid)
-    int min_rows = 1024;    // smallest tile (four rows per thread of a 256-thread block)
-    int per_sm = 4;         // cap of the cooperative grid in blocks per SM
+    int tiles = 296;        // tiles of a large member (two per SM)
+    int min_rows = 256;     // smallest tile: a 30k-row member still reaches most SMs (mixed-precision solve
+                            // 2.4 ms, against 2.7 with 1,024-row tiles; 1M rows the same)
 };
 struct LaunchTable {
     // the node gathers (nodal velocities, nodal tracers) at 512 threads: the tuner's choice on
@@ -108,7 +109,10 @@ struct Dev {
     int2* sell;
     int32_t *indices;
     double *A;
-    float *A32;                    // D^-1 A in FP32 (refinement solve)
+    // refinement solve: FP32 D^-1 A off the diagonal in ball order (null in FP64 contexts) and the
+    // position of each row's entry 0 in it
+    float *A32;
+    int32_t *row_at32;
     // JCG vectors
     double *b, *xs, *r, *zz, *p0, *p1, *q, *invD, *xh0, *xh1, *xh2;
     float *ir32, *diag32;          // ir32: kIrVectors FP32 vectors of the refinement solve

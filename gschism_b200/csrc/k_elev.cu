@@ -248,19 +248,18 @@ __global__ void k_assemble(Dev d, Phys P) {
                 }
             }
         }
-        // FP64 row, and the row of D^-1 A in FP32 for the refinement solve
+        // FP64 row, and the row of D^-1 A in FP32 (one line per slot) for the refinement solve
         const double inv = 1.0 / diag;
-        for (int p = 0; p < nn; p++) {
-            const int at = d.nbr_slot[s0 + p];
-            d.A[at] = vals[p];
-            d.A32[at] = (float)(vals[p] * inv);
-        }
+        for (int p = 0; p < nn; p++) d.A[d.nbr_slot[s0 + p]] = vals[p];
         d.A[d.diag_slot[i]] = diag;
-        d.A32[d.diag_slot[i]] = 1.0f;
+        if (d.A32) {
+            const size_t at = d.row_at32[i];
+            for (int p = 0; p < nn; p++) d.A32[at + 32 * (size_t)p] = (float)(vals[p] * inv);
+            d.diag32[i] = (float)diag;
+        }
         d.qel[i] = qel;
         d.b[i] = qel;
         d.invD[i] = inv;
-        d.diag32[i] = (float)diag;
         d.xs[i] = 3.0 * d.xh0[i] - 3.0 * d.xh1[i] + d.xh2[i];
     }
 }

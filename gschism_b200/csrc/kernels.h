@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "gs_internal.h"
+#include "mg.h"
 
 namespace gs {
 
@@ -20,6 +21,7 @@ struct JcgArgs {
     double *x, *r, *z, *q, *p0, *p1;
     float* ir32;                         // kIrVectors * n floats
     const float* diag32;                 // matrix diagonal in FP32
+    const MgDev* mg;                     // hierarchy of a context's refinement solve
     unsigned* bar;
     int32_t* err;
     double rtol;

@@ -1,0 +1,63 @@
+// Multilevel hierarchy of the FP32 refinement solve (jcg_mg.cu): layout, host construction
+// (mg_setup.cpp) and launch.
+#pragma once
+#include <cstdint>
+#include <vector>
+
+#include <vector_types.h>
+
+namespace gs {
+
+constexpr int kMgLevels = 4;          // coarse levels; level k joins 4^k consecutive rows of a member
+constexpr int kMgChunk = 256;         // a member's coarse rows start at a multiple of this on level 1
+constexpr int kMgPad = 2048;          // level-1 rows of the batch, so that every level has whole slices
+constexpr uint8_t kMgDiag = 255;      // Galerkin map: the entry falls inside its own aggregate
+constexpr int kMgMaxSlots = 255;      // widest coarse row
+
+// FP32 matrices without their (unit) diagonal in SELL-32: entry k of row l of slice s sits at
+// sl[s].x + 32 k + l for k < sl[s].y; padding entries hold the row itself and a zero value.
+struct MgMatrix {
+    int2* sl = nullptr;
+    int32_t* idx = nullptr;
+    float* val = nullptr;             // D^-1 A off the diagonal
+    uint8_t* map = nullptr;           // slot of the entry in its aggregate's row one level up
+};
+struct MgLevel {
+    int n = 0;                        // rows (a multiple of 32; rows of no aggregate stay zero)
+    MgMatrix A;
+    float *D = nullptr, *Dinv = nullptr;
+    float *rh = nullptr;              // D^-1 (restricted residual)
+    float *e = nullptr;               // correction
+};
+struct MgDev {
+    MgMatrix A;                       // fine matrix, slices relative to the member's first row
+    MgLevel lv[kMgLevels];
+    float *cr = nullptr, *cd = nullptr;   // coarsest level: residual and last step of the polynomial
+    int32_t *mem_s = nullptr;         // [nmem] a member's first fine slice
+    int32_t *mem_c = nullptr;         // [nmem] a member's first row on level 1, -1: no hierarchy
+    int32_t *chunk_mem = nullptr;     // [level-1 rows / kMgChunk] member, -1 padding
+    int2 *chunk_fine = nullptr;       // first fine row of the chunk and the number of fine rows under it
+    int32_t *row_at = nullptr;        // [rows] position of a row's entry 0 in A
+};
+
+// Host side: structure of every level of a batch.
+struct MgHostMatrix {
+    std::vector<int2> sl;
+    std::vector<int32_t> idx;
+    std::vector<uint8_t> map;
+};
+struct MgHost {
+    MgHostMatrix A, lv[kMgLevels];
+    int n[kMgLevels] = {0};
+    std::vector<int32_t> mem_s, mem_c, chunk_mem, row_at;
+    std::vector<int2> chunk_fine;
+};
+// Members with fewer rows use plain Jacobi (no hierarchy).
+constexpr int kMgMinRows = 4096;
+// nnp_s/nnp: node -> nodes of the batch (global rows, ball order); row0/rows per member.
+// Returns false when a matrix needs more than 32-bit offsets or a coarse row has more neighbours
+// than a map byte can name; without `levels` no member gets a hierarchy.
+bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const std::vector<int32_t>& nnp_s,
+              const std::vector<int32_t>& nnp, bool levels, MgHost& H);
+
+}  // namespace gs

@@ -61,6 +61,7 @@ struct Prepared {
     std::vector<ElemGeo> egeo;            // [NE]
     std::vector<int2> sell;               // SELL-32 slices
     std::vector<int32_t> sidx;            // SELL entries' columns
+    MgHost mg;                            // hierarchy of the refinement solve (GS_FP32_IR)
 };
 
 }  // namespace
@@ -77,6 +78,7 @@ struct gs_ctx {
     VG vg{};
     Phys P{};
     JcgWork* jw = nullptr;
+    MgDev mg{};
     std::vector<void*> allocs;
     int it = 0;
     // gs_step replays one captured step; recaptured when storm forcing switches on or off
@@ -495,6 +497,12 @@ static gs_status prepare_host(gs_ctx* c) {
         c->h_indptr = B.indptr;
         c->h_indices = B.indices;
     }
+    if (c->cfg.precision == GS_FP32_IR) {
+        std::vector<int> row0, rows;
+        for (auto& m : c->mem) { row0.push_back(m.np0); rows.push_back(m.np); }
+        if (!mg_build(row0, rows, B.nnp_s, B.nnp, true, pr->mg) && !mg_build(row0, rows, B.nnp_s, B.nnp, false, pr->mg))
+            return c->fail(GS_ERR_ARG, "elevation matrix too large for 32-bit offsets");
+    }
     c->prep = guard.release();
     return GS_OK;
 }
@@ -558,10 +566,47 @@ extern "C" gs_status gs_ctx_finalize(gs_ctx* c) {
     UP(nbr_slot, B.nbr_slot); UP(diag_slot, B.diag_slot); UP(sb1, B.sb1); UP(sb2, B.sb2);
     UP(bn_node, B.bn_node); UP(bn_ietype, B.bn_ietype); UP(bn_nbfr, B.bn_nbfr);
     UP(bn_emo, B.bn_emo); UP(bn_efa, B.bn_efa); UP(bn_amig, B.bn_amig); UP(bn_ff, B.bn_ff); UP(bn_face, B.bn_face);
-    UP(sell, sell); UP(indices, sidx); AL(A, d.NNZ); AL(A32, d.NNZ);
+    UP(sell, sell); UP(indices, sidx); AL(A, d.NNZ);
     AL(b, NP); AL(xs, NP); AL(r, NP); AL(zz, NP); AL(p0, NP); AL(p1, NP); AL(q, NP); AL(invD, NP);
     AL(xh0, NP); AL(xh1, NP); AL(xh2, NP);
-    AL(ir32, (size_t)kIrVectors * NP); AL(diag32, NP);
+    if (c->cfg.precision == GS_FP32_IR) {
+        AL(ir32, (size_t)kMgVectors * NP); AL(diag32, NP);
+        // the hierarchy's arrays share one allocation
+        const MgHost& H = pr->mg;
+        MgDev& g = c->mg;
+        std::vector<unsigned char> img;       // host image of the uploaded arrays, at their offsets
+        size_t bytes = 0;
+        std::vector<std::pair<void**, size_t>> at;
+        auto room = [&](auto*& p, size_t n) {
+            at.push_back({(void**)&p, bytes});
+            bytes += (n * sizeof(*p) + 255) / 256 * 256;
+        };
+        auto put = [&](auto*& p, const auto& h) {
+            room(p, h.size());
+            img.resize(bytes);
+            if (!h.empty()) std::memcpy(img.data() + at.back().second, h.data(), h.size() * sizeof(h[0]));
+        };
+        put(g.A.sl, H.A.sl); put(g.A.idx, H.A.idx); put(g.A.map, H.A.map);
+        for (int k = 0; k < kMgLevels; k++) {
+            g.lv[k].n = H.n[k];
+            put(g.lv[k].A.sl, H.lv[k].sl); put(g.lv[k].A.idx, H.lv[k].idx); put(g.lv[k].A.map, H.lv[k].map);
+        }
+        put(g.mem_s, H.mem_s); put(g.mem_c, H.mem_c); put(g.chunk_mem, H.chunk_mem); put(g.chunk_fine, H.chunk_fine);
+        put(g.row_at, H.row_at);
+        room(g.A.val, H.A.idx.size());
+        for (int k = 0; k < kMgLevels; k++) {
+            MgLevel& L = g.lv[k];
+            room(L.A.val, H.lv[k].idx.size());
+            room(L.D, L.n); room(L.Dinv, L.n); room(L.rh, L.n); room(L.e, L.n);
+        }
+        room(g.cr, H.n[kMgLevels - 1]); room(g.cd, H.n[kMgLevels - 1]);
+        unsigned char* base = nullptr;
+        if (e == cudaSuccess) e = dalloc(c, base, bytes);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(base, img.data(), img.size(), cudaMemcpyHostToDevice, c->own_st);
+        for (auto& q : at) *q.first = base + q.second;
+        d.A32 = g.A.val;
+        d.row_at32 = g.row_at;
+    }
     UP(sn, B.sn); UP(se, B.se); UP(len, B.len); UP(snx, B.snx); UP(sny, B.sny); UP(scx, B.scx); UP(scy, B.scy);
     UP(cori, B.cori); AL(kbs, NS); AL(sdry, NS); UP(sbt, B.sbt);
     AL(zc, (size_t)nvrt * NS); AL(Qh, (size_t)nvrt * NS); AL(su2, (size_t)nvrt * NS); AL(btu, (size_t)nvrt * NS);
@@ -636,7 +681,7 @@ static gs_status run_phase(gs_ctx* c, int phase, int arg) {
         JcgArgs a{};
         Dev& d = c->d;
         a.n = d.NP; a.precision = c->cfg.precision;
-        a.indptr = nullptr; a.sell = d.sell; a.indices = d.indices; a.A = d.A; a.A32 = d.A32; a.b = d.b; a.invD = d.invD;
+        a.indptr = nullptr; a.sell = d.sell; a.indices = d.indices; a.A = d.A; a.A32 = nullptr; a.mg = &c->mg; a.b = d.b; a.invD = d.invD;
         a.x = d.xs; a.r = d.r; a.z = d.zz; a.q = d.q; a.p0 = d.p0; a.p1 = d.p1;
         a.ir32 = d.ir32; a.diag32 = d.diag32;
         a.bar = d.bar; a.err = d.err;
@@ -812,8 +857,7 @@ gs_status gs_set_launch(gs_ctx* c, int kernel, int a, int b) {
     if (!c || !c->finalized || kernel < 0 || kernel > GS_K_JCG_TILES) return GS_ERR_ARG;
     cudaSetDevice(c->dev);
     if (kernel == GS_K_JCG_TILES) {
-        // a = tiles of a large member, b = smallest tile (rows, a multiple of 32); the cap of the
-        // cooperative grid stays at its default
+        // a = tiles of a large member, b = smallest tile (rows, a multiple of 32)
         if (a < 1 || a > 65536 || b < 32 || b > (1 << 24) || b % 32 != 0) return GS_ERR_ARG;
         JcgTiling tl = c->launch.jcg;
         tl.tiles = a; tl.min_rows = b;
@@ -1257,6 +1301,11 @@ extern "C" size_t gs_footprint_bytes(int nvrt, int ntr, int nmem, int64_t np, in
     b += (double)ns * (16.0 + 70.0 + 72.0 + 16.0 + 48.0 + L * 52.0 + 4.0);
     b += std::max(L * 16.0 * (double)ns, L * 8.0 * T * (double)ne);   // field exchange staging (largest field)
     b += sell * 16.0 + (double)np / 32.0 * 8.0;
+    // refinement solve: fine FP32 matrix, and the coarse levels (a third of the rows, each member
+    // rounded up to whole chunks, up to 16 entries a row)
+    const double coarse = ((double)np / 4.0 + (double)nmem * kMgChunk + kMgPad) * 4.0 / 3.0;
+    b += ((double)std::max<int64_t>(nnz - np, 0) * 1.25 + 32.0 * kMaxDeg * nmem) * 9.0 + (double)np * 4.0 +
+         ((double)np / 32.0 + nmem) * 8.0 + coarse * (16.0 * 9.0 + 28.0);
     b += ((double)np / 1024.0 + nmem) * 84.0 + (double)nmem * (16.0 + 72.0 + 40.0 + 8.0 * kVortexParams + 64.0 + 8.0);
     b += (double)kMassBlocks * kMaxTracers * 16.0 + kMaxTracers * 8.0;
     b += 256.0 * 1024 * 1024;                   // allocation granularity of ~120 allocations

@@ -1,0 +1,101 @@
+"""The elevation solves at the edges of their forms: the mixed-precision solve with its aggregation
+hierarchy (jcg_mg.cu) against the FP64 oracle, members alone and in batches (gpu).
+
+Sizes: both sides of the 4,096-row line between plain Jacobi and the hierarchy, and row counts that
+are no multiple of an aggregate (4), a slice (32) or a chunk of 1,024 rows.  A Delaunay mesh of random
+points has nodes with more than eight neighbours, whose slices are read past the shared-memory ring.
+
+Bound: a solve stops at |b - A x| <= 1e-12 |b|; the mass matrix bounds A from below by the smallest
+element areas, and measured against the FP64 oracle the elevations of these meshes differ by less
+than 1e-11 of the largest one after a step, so 1e-9 leaves two digits for three steps."""
+import numpy as np
+import pytest
+
+from gschism_b200 import cases
+from tests._parity import relerr
+
+pytestmark = pytest.mark.gpu
+
+
+def _basin(seed, side):
+    c = cases.basin(seed=seed, n=side, nvrt=4, nz=2, ntr=1, length=500.0 * side)
+    c.params.dramp = 0.05
+    return c
+
+
+def _delaunay(seed, side):
+    """A basin of the same outline on random interior points (node degrees 3 to about 12)."""
+    spatial = pytest.importorskip("scipy.spatial")
+    c = _basin(seed, side)
+    rng = np.random.default_rng(seed)
+    length = 500.0 * side
+    bnd = np.unique(np.concatenate(c.open_bnd + c.land_bnd))
+    inner = np.setdiff1d(np.arange(c.n_nodes), bnd)
+    lo, hi = 250.0, length - 250.0
+    c.x[inner], c.y[inner] = rng.uniform(lo, hi, inner.size), rng.uniform(lo, hi, inner.size)
+    # the outline bulges slightly, so that every boundary node is a corner of the hull
+    bx, by = c.x[bnd] / length - 0.5, c.y[bnd] / length - 0.5
+    sx, sy = np.abs(bx) >= np.abs(by), np.abs(by) >= np.abs(bx)
+    c.x[bnd] += np.where(sx, np.sign(bx) * 100.0 * (0.25 - by ** 2), 0.0)
+    c.y[bnd] += np.where(sy, np.sign(by) * 100.0 * (0.25 - bx ** 2), 0.0)
+    tri = spatial.Delaunay(np.stack([c.x, c.y], 1)).simplices
+    a, b, d = (np.stack([c.x[tri[:, k]], c.y[tri[:, k]]], 1) for k in range(3))
+    ccw = (b[:, 0] - a[:, 0]) * (d[:, 1] - a[:, 1]) - (d[:, 0] - a[:, 0]) * (b[:, 1] - a[:, 1]) > 0
+    tri = np.where(ccw[:, None], tri, tri[:, ::-1])
+    c.elnode = np.ascontiguousarray(tri, dtype=np.int32)
+    deg = np.bincount(c.elnode.ravel(), minlength=c.n_nodes)
+    assert deg.max() > 8
+    return c
+
+
+@pytest.mark.parametrize("make", [lambda: _basin(11, 63), lambda: _basin(12, 64), lambda: _basin(13, 65),
+                                  lambda: _basin(14, 101), lambda: _delaunay(15, 80)],
+                         ids=["3969", "4096", "4225", "10201", "delaunay6400"])
+def test_elevation_against_oracle(native, oracle_lib, make):
+    from gschism_b200.model import Model
+    from oracle.step_api import OracleModel
+    c = make()
+    o = OracleModel(c)
+    o.run(3)
+    g = Model([c], precision="fp32_ir")
+    g.step(3)
+    st = g.stats(0)
+    assert st["error_flags"] == 0
+    assert relerr(g.get(0, "ETA2"), o.get("ETA2")) <= 1e-9
+    g.close()
+
+
+@pytest.mark.parametrize("tiles", [None, (40, 32)])
+def test_members_equal_their_solo_runs(native, tiles):
+    """Members on both sides of the line, and one with wide rows, in one context: bit for bit the
+    results of each member alone, with the default tiles and with 32-row ones."""
+    from gschism_b200.model import Model
+    cs = [_basin(21, 40), _delaunay(22, 70), _basin(23, 101), _basin(24, 66)]
+    mix = Model(cs, precision="fp32_ir")
+    if tiles:
+        mix.set_launch("JCG_TILES", *tiles)
+    mix.step(3)
+    for k, c in enumerate(cs):
+        solo = Model([c], precision="fp32_ir")
+        if tiles:
+            solo.set_launch("JCG_TILES", *tiles)
+        solo.step(3)
+        assert np.array_equal(mix.get(k, "ETA2"), solo.get(0, "ETA2")), k
+        assert mix.stats(k)["jcg_iters"] == solo.stats(0)["jcg_iters"]
+        solo.close()
+    mix.close()
+
+
+def test_fp64_member_in_a_batch_beyond_shared_memory(native):
+    """The FP64 solve holds the matrix in shared memory while it fits; a batch of more rows reads it
+    from global memory with other launch shapes.  A member gets the same bits in both."""
+    from gschism_b200.model import Model
+    cs = [_basin(31, 45), _basin(32, 640)]
+    mix = Model(cs, precision="fp64", maxiter=60)
+    solo = Model(cs[:1], precision="fp64", maxiter=60)
+    mix.step(2)
+    solo.step(2)
+    assert np.array_equal(mix.get(0, "ETA2"), solo.get(0, "ETA2"))
+    assert mix.stats(0)["jcg_iters"] == solo.stats(0)["jcg_iters"]
+    mix.close()
+    solo.close()
