@@ -139,8 +139,6 @@ struct Dev {
     double *ez, *ew, *Qv;          // [nvrt][NE]
     double *etr, *prev;            // [ntr][nvrt][NE]
     double *tvds;                  // [ntr][nvrt][NE] TVD inflow sums (allocated with TVD only)
-    double *vgam;                  // [nvrt][NE] vertical sweep scratch (allocated with vertical FCT only)
-    double *maxDt;
     double2 *ghat;
     double *rho_n, *rho_e;         // [nvrt][NP], [nvrt][NE] densities (allocated with >= 2 tracers)
     // members
