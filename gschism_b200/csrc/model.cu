@@ -618,8 +618,7 @@ extern "C" gs_status gs_ctx_finalize(gs_ctx* c) {
     AL(ez, (size_t)nvrt * NE); AL(ew, (size_t)nvrt * NE); AL(Qv, (size_t)nvrt * NE);
     UP(etr, B.etr); AL(prev, (size_t)ntr * nvrt * NE);
     if (c->cfg.itr_met >= 3) AL(tvds, (size_t)ntr * nvrt * NE);
-    if (c->cfg.itr_met == 4) AL(vgam, (size_t)nvrt * NE);
-    AL(maxDt, NE); AL(ghat, NE);
+    AL(ghat, NE);
     if (ntr >= 2) { AL(rho_n, (size_t)nvrt * NP); AL(rho_e, (size_t)nvrt * NE); }
     UP(mem_np0, B.mem_np0); UP(mem_ne0, B.mem_ne0); UP(elem_member, B.elem_member);
     c->h_vort.assign((size_t)kVortexParams * c->mem.size(), 0.0);
