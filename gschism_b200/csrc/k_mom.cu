@@ -51,7 +51,10 @@ __device__ __forceinline__ double2 slip(double2 u, int8_t bt, double nx, double 
     return t * vtan - nn * vnorm;
 }
 
-__global__ void __launch_bounds__(128, 8) k_momentum(Dev d, Phys P) {
+// Bound by the latency of a column's level loop (divisions that depend on the level below, and loads).  Each
+// level's inputs are loaded one level ahead of its divisions; at four blocks of 128 per SM that needs no
+// spills: 742 us on 1.08M sides of 30 levels, 892 without the loads ahead at eight blocks (with them 1,052).
+__global__ void __launch_bounds__(128, 4) k_momentum(Dev d, Phys P) {
     const int NS = d.NS, nvrt = P.nvrt;
     const double dt = P.dt, th = P.thetai;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < NS; s += gridDim.x * blockDim.x) {
@@ -97,11 +100,19 @@ __global__ void __launch_bounds__(128, 8) k_momentum(Dev d, Phys P) {
             double zkm1 = d.zc[(size_t)kb * NS + s], zk = d.zc[(size_t)(kb + 1) * NS + s];
             double bet = 0.0, cprev = 0.0;
             double2 rprev = v2(0.0, 0.0);
+            // level k + 1, and what level k + 2 holds, loaded ahead of level k's divisions
+            const bool two = kb + 2 < nvrt;
+            double2 ukp1 = two ? u2[(size_t)(kb + 2) * NS + s] : v2(0.0, 0.0);
+            double2 bkp1 = two ? btu[(size_t)(kb + 2) * NS + s] : v2(0.0, 0.0);
+            double zkp1 = two ? d.zc[(size_t)(kb + 2) * NS + s] : 0.0;
             for (int k = kb + 1; k < nvrt; k++) {
                 const bool top = (k == nvrt - 1);
-                const double2 ukp1 = top ? v2(0.0, 0.0) : u2[(size_t)(k + 1) * NS + s];
-                const double2 bkp1 = top ? v2(0.0, 0.0) : btu[(size_t)(k + 1) * NS + s];
-                const double zkp1 = top ? 0.0 : d.zc[(size_t)(k + 1) * NS + s];
+                double2 ukp2 = v2(0.0, 0.0), bkp2 = v2(0.0, 0.0);
+                double zkp2 = 0.0;
+                if (k + 2 < nvrt) {
+                    const size_t ix = (size_t)(k + 2) * NS + s;
+                    ukp2 = u2[ix]; bkp2 = btu[ix]; zkp2 = d.zc[ix];
+                }
                 double alow = 0.0, cupp = 0.0, bdia = 0.0;
                 const double cff1 = 1.0;
                 const double dz_0 = zk - zkm1;
@@ -148,25 +159,29 @@ __global__ void __launch_bounds__(128, 8) k_momentum(Dev d, Phys P) {
                 u2[(size_t)k * NS + s] = r;
                 rprev = r;
                 cprev = cupp;
-                ukm1 = uk; uk = ukp1; bkm1 = bk; bk = bkp1; zkm1 = zk; zk = zkp1;
+                ukm1 = uk; uk = ukp1; ukp1 = ukp2; bkm1 = bk; bk = bkp1; bkp1 = bkp2; zkm1 = zk; zk = zkp1; zkp1 = zkp2;
             }
             rtop = rprev;
         }
         // top-down: back substitution (3D), clamp, the bottom level's value, free slip on land
         // sides, and the stores of u2 and of the fluxes Qh (land sides carry zero flux)
-        double2 r = rtop, uabove = v2(0.0, 0.0);
-        double zabove = 0.0;
+        // (the next level down is loaded ahead)
+        double2 r = rtop, uabove = v2(0.0, 0.0), xn = v2(0.0, 0.0);
+        double zabove = 0.0, gn = 0.0, zn = d.zc[(size_t)(nvrt - 1) * NS + s];
         for (int k = nvrt - 1; k >= kb; k--) {
+            const double2 x = xn;
+            const double gam = gn, zk = zn;
+            if (k > kb) {
+                const size_t ix = (size_t)(k - 1) * NS + s;
+                zn = d.zc[ix];
+                if (!two_d && k - 1 > kb) { xn = u2[ix]; gn = Qh[ix + NS]; }
+            }
             double2 u;
             if (k > kb) {
                 if (two_d) {
                     u = vel2d;
                 } else {
-                    if (k < nvrt - 1) {
-                        const double gam = Qh[(size_t)(k + 1) * NS + s];
-                        const double2 x = u2[(size_t)k * NS + s];
-                        r = v2(x.x - gam * r.x, x.y - gam * r.y);
-                    }
+                    if (k < nvrt - 1) r = v2(x.x - gam * r.x, x.y - gam * r.y);
                     u = clampvel(r, P.rmaxvel);
                 }
             } else {
@@ -176,7 +191,6 @@ __global__ void __launch_bounds__(128, 8) k_momentum(Dev d, Phys P) {
             }
             u = slip(u, bt, nx, ny);
             u2[(size_t)k * NS + s] = u;
-            const double zk = d.zc[(size_t)k * NS + s];
             if (k < nvrt - 1)
                 Qh[(size_t)(k + 1) * NS + s] = (bt == 1) ? 0.0 : side_flux(len, nx, ny, zabove, zk, uabove, u);
             uabove = u;
@@ -187,7 +201,10 @@ __global__ void __launch_bounds__(128, 8) k_momentum(Dev d, Phys P) {
     }
 }
 
-__global__ void __launch_bounds__(128, 6) k_vvel(Dev d, Phys P) {
+// Bound by the latency of the level loop, as k_momentum: a side's values are read once and carried to the
+// next level, and the next level's are loaded ahead.  343 us on 720k elements of 30 levels at four blocks
+// per SM (371 at three, 564 with spills at six), 508 with both levels read at every step.
+__global__ void __launch_bounds__(128, 4) k_vvel(Dev d, Phys P) {
     // computeVerticalVelocity, meshdata.cu:5978-6103 (imm = 0, triangles, ics = 1)
     const int NE = d.NE, NS = d.NS, NP = d.NP, nvrt = P.nvrt;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < NE; e += gridDim.x * blockDim.x) {
@@ -211,11 +228,34 @@ __global__ void __launch_bounds__(128, 6) k_vvel(Dev d, Phys P) {
         const double x0 = d.x[n0], y0 = d.y[n0], x1 = d.x[n1], y1 = d.y[n1], x2 = d.x[n2], y2 = d.y[n2];
         const int kb0 = d.kb[n0], kb1 = d.kb[n1], kb2 = d.kb[n2];
         const double az = 2.0 * d.area[e];
+        // A side's velocity and height on levels l (held from the level before), l + 1 and, loaded ahead of
+        // level l's square root and divisions, l + 2; the corners' heights likewise
+        int kbs[3];
+        double2 ulo[3], uhi[3];
+        double zlo[3], zhi[3], wn[3];
+        for (int j = 0; j < 3; j++) {
+            const int s = sd[j];
+            kbs[j] = d.kbs[s];
+            const int ka = max(min(kb + 1, nvrt - 1), kbs[j]), kc = max(kb, kbs[j]);
+            ulo[j] = d.su2[(size_t)kc * NS + s]; zlo[j] = d.zc[(size_t)kc * NS + s];
+            uhi[j] = d.su2[(size_t)ka * NS + s]; zhi[j] = d.zc[(size_t)ka * NS + s];
+            wn[j] = (double)d.ssgn[j * NE + e];
+        }
+        const int nd[3] = {n0, n1, n2}, kbn[3] = {kb0, kb1, kb2};
+        double zn[3];
+        for (int j = 0; j < 3; j++) zn[j] = d.z[(size_t)max(min(kb + 1, nvrt - 1), kbn[j]) * NP + nd[j]];
         for (int l = kb; l < nvrt - 1; l++) {
-            const int k = l + 1;
-            const double z0 = d.z[(size_t)(k > kb0 ? k : kb0) * NP + n0];
-            const double z1 = d.z[(size_t)(k > kb1 ? k : kb1) * NP + n1];
-            const double z2 = d.z[(size_t)(k > kb2 ? k : kb2) * NP + n2];
+            const double z0 = zn[0], z1 = zn[1], z2 = zn[2];
+            double2 unx[3];
+            double znx[3];
+            {
+                const int k2 = min(l + 2, nvrt - 1);
+                for (int j = 0; j < 3; j++) {
+                    const size_t ka = max(k2, kbs[j]);
+                    unx[j] = d.su2[ka * NS + sd[j]]; znx[j] = d.zc[ka * NS + sd[j]];
+                    zn[j] = d.z[(size_t)max(k2, kbn[j]) * NP + nd[j]];
+                }
+            }
             const double n20x = x2 - x0, n20y = y2 - y0, n20z = z2 - z0;
             const double n10x = x1 - x0, n10y = y1 - y0, n10z = z1 - z0;
             const double ax = n10y * n20z - n20y * n10z;
@@ -228,19 +268,12 @@ __global__ void __launch_bounds__(128, 6) k_vvel(Dev d, Phys P) {
             double2 um = v2(0.0, 0.0);
             for (int j = 0; j < 3; j++) {
                 const int s = sd[j];
-                const int kbs = d.kbs[s];
-                const int ka = (l + 1 > kbs) ? l + 1 : kbs, kc = (l > kbs) ? l : kbs;
-                const double2 ut = d.su2[(size_t)ka * NS + s], ubt = d.su2[(size_t)kc * NS + s];
-                const double2 u2c = (ut + ubt) * 0.5;
-                const double sideArea = d.len[s] * (d.zc[(size_t)ka * NS + s] - d.zc[(size_t)kc * NS + s]);
-                const double sign = (double)d.ssgn[j * NE + e];
-                sideFlux += sign * (u2c.x * d.snx[s] + u2c.y * d.sny[s]) * sideArea;
+                const double2 u2c = (uhi[j] + ulo[j]) * 0.5;
+                const double sideArea = d.len[s] * (zhi[j] - zlo[j]);
+                sideFlux += wn[j] * (u2c.x * d.snx[s] + u2c.y * d.sny[s]) * sideArea;
             }
-            for (int j = 0; j < 3; j++) {
-                const int s = sd[j];
-                const int kk = (l + 1 > d.kbs[s]) ? l + 1 : d.kbs[s];
-                um = um + d.su2[(size_t)kk * NS + s];
-            }
+            for (int j = 0; j < 3; j++) um = um + uhi[j];
+            for (int j = 0; j < 3; j++) { ulo[j] = uhi[j]; zlo[j] = zhi[j]; uhi[j] = unx[j]; zhi[j] = znx[j]; }
             um = (um + v2(0.0, 0.0)) / 3;
             const double topFlux = -sideFlux - bottomFlux;
             d.Qv[(size_t)(l + 1) * NE + e] = topFlux;
