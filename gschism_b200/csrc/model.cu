@@ -1039,9 +1039,10 @@ gs_status field_block(gs_ctx* c, const MemberHost& m, const FieldInfo& fi, size_
     return GS_OK;
 }
 
-// Staging blocks of at least `bytes`: the device block and the next pinned host block (after its
-// previous copy has finished).  Grows them on demand.
-cudaError_t stage(gs_ctx* c, size_t bytes, int& h) {
+// Staging blocks of at least `bytes`: the device block and, for a copy that goes through it (`host`), the
+// next pinned host block (after its previous copy has finished).  Grows them on demand; page-locked
+// caller memory needs no host block, whose allocation costs 5 to 90 ms on a context's first exchange.
+cudaError_t stage(gs_ctx* c, size_t bytes, bool host, int& h) {
     cudaError_t e = cudaSuccess;
     if (c->dstage_bytes < bytes) {
         if (c->dstage) { cudaStreamSynchronize(c->st); cudaFree(c->dstage); }
@@ -1059,7 +1060,7 @@ cudaError_t stage(gs_ctx* c, size_t bytes, int& h) {
         e = cudaEventSynchronize(c->hev[h]);
         if (e != cudaSuccess) return e;
     }
-    if (c->hstage_bytes[h] < bytes) {
+    if (host && c->hstage_bytes[h] < bytes) {
         if (c->hstage[h]) cudaFreeHost(c->hstage[h]);
         c->hstage[h] = nullptr; c->hstage_bytes[h] = 0;
         e = cudaHostAlloc(&c->hstage[h], bytes, cudaHostAllocDefault);
@@ -1081,9 +1082,9 @@ bool page_locked(const void* p) {
 // scatter run on the context stream either way.
 cudaError_t put_block(gs_ctx* c, const void* host, size_t bytes, void* dst, const Block& k) {
     int h = 0;
-    cudaError_t e = stage(c, bytes, h);
-    if (e != cudaSuccess) return e;
     const bool direct = page_locked(host);
+    cudaError_t e = stage(c, bytes, !direct, h);
+    if (e != cudaSuccess) return e;
     if (!direct) std::memcpy(c->hstage[h], host, bytes);
     e = cudaMemcpyAsync(c->dstage, direct ? host : c->hstage[h], bytes, cudaMemcpyHostToDevice, c->st);
     if (e != cudaSuccess) return e;
@@ -1131,12 +1132,12 @@ extern "C" gs_status gs_state_get(gs_ctx* c, int member, int field, void* host, 
     gs_status st = field_block(c, m, fi, bytes, k);
     if (st != GS_OK) return st;
     int h = 0;
-    cudaError_t e = stage(c, bytes, h);
+    // page-locked destinations take the copy directly, others through pinned staging
+    const bool direct = page_locked(host);
+    cudaError_t e = stage(c, bytes, !direct, h);
     if (e != cudaSuccess) return c->fail(GS_ERR_CUDA, cudaGetErrorString(e));
     launch_gather(fi.ptr, c->dstage, k.kind, k.n, k.N, k.off, k.nslices, k.nc, k.perm,
                   field == GS_F_SIDE_BTELEM ? c->d.pe_ref : nullptr, c->st, c->nsm);
-    // page-locked destinations take the copy directly, others through pinned staging
-    const bool direct = page_locked(host);
     e = cudaMemcpyAsync(direct ? host : c->hstage[h], c->dstage, bytes, cudaMemcpyDeviceToHost, c->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
     if (e != cudaSuccess) return c->fail(GS_ERR_CUDA, cudaGetErrorString(e));
