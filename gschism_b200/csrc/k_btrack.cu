@@ -41,13 +41,17 @@ __device__ unsigned valid_exits(const ElemGeo* geo, int e, double2 x0, double2 x
     const double2 vt0 = xt - x0;
     double mp = fmax(dot2(vt0, C[0] - x0), dot2(vt0, C[1] - x0));
     mp = fmax(mp, dot2(vt0, C[2] - x0));
-    fac = fmax(1.00001 * fac, fmin(1.0, (mp / dot2(vt0, vt0)) * 1.00001));
+    // min(1, (mp / |vt0|^2) 1.00001): 1 whenever mp reaches |vt0|^2, which it does unless the target lies
+    // near or beyond the farthest corner, so the division is rarely made
+    const double vv = dot2(vt0, vt0);
+    fac = fmax(1.00001 * fac, mp >= vv ? 1.0 : fmin(1.0, (mp / vv) * 1.00001));
     const double2 ixt = x0 + (xt - x0) * fac;
     const double2 s0 = C[1] - C[0], s1 = C[2] - C[1], s2 = C[0] - C[2];
     unsigned left = 0u, bis = 0u;
     left |= (unsigned)(cross2(s0, ixt - C[0]) > -kSmall);
     left |= (unsigned)(cross2(s1, ixt - C[1]) > -kSmall) << 1;
     left |= (unsigned)(cross2(s2, ixt - C[2]) > -kSmall) << 2;
+    if (left == 7u) return 0u;       // inside: the exits are not needed
     const unsigned obt = (unsigned)(pm >> 8) & 7u;
     bis |= (unsigned)(dot2(ixt - C[1], s0 + s1) < 0.0);
     bis |= (unsigned)(dot2(ixt - C[2], s1 + s2) < 0.0) << 1;
