@@ -41,7 +41,7 @@ TUNE_ORDER = ["BTRACK", "JCG_TILES", "MOMENTUM", "SIDE_PREP", "GHAT", "VVEL", "N
 def candidates(kernel: str) -> List[Shape]:
     """Shapes tried for a kernel (the library rejects those its compiled kernel cannot run)."""
     if kernel == "JCG_TILES":
-        return [(592, 1024), (296, 1024), (444, 1024), (888, 1024), (1184, 512), (888, 512)]
+        return [(296, 256), (148, 256), (592, 256), (592, 1024), (296, 1024), (444, 1024), (888, 1024), (1184, 512), (888, 512)]
     return [(b, g) for b in (64, 128, 256, 512) for g in (16, 32)]
 
 

@@ -64,10 +64,8 @@ struct JcgTiling {
                             // 2.4 ms, against 2.7 with 1,024-row tiles; 1M rows the same)
 };
 struct LaunchTable {
-    // the node gathers (nodal velocities, nodal tracers) at 512 threads: the tuner's choice on
-    // both the 1M basin and the 64-member ensemble (nodal velocities 20% faster than at 128)
     LaunchShape k[LK_COUNT] = {{128, 32}, {256, 16}, {256, 16}, {128, 16}, {128, 32},
-                               {128, 32}, {512, 32}, {512, 16}, {256, 16}};
+                               {128, 32}, {256, 32}, {256, 16}, {256, 16}};
     JcgTiling jcg;
 };
 
@@ -149,12 +147,6 @@ struct Dev {
     double *mem_rem, *mem_dtb;     // transport sub-cycling per member
     unsigned long long *mem_mindt; // positive doubles ordered as unsigned
     int32_t *mem_nsub;
-    // JCG work list: tiles of rows inside one member
-    int ntiles;
-    int32_t *tile_r0, *tile_r1, *tile_mem, *mem_t0, *mem_t1;
-    double *tile_part;             // [4][ntiles] partial sums
-    double *mem_scal;              // per member scalars (see jcg.cu)
-    int32_t *mem_iters, *mem_outer;
     // global control
     double* clk;                   // [3] step, time = step * dt, ramp (set on the device each step)
     unsigned* bar;                  // grid barrier word (zero between launches)

@@ -232,8 +232,8 @@ void launch_nodal_vel(const Dev& d, const Phys& P, cudaStream_t st, int nsm, con
 
 int levels_max_threads(int kernel) {
     cudaFuncAttributes a{};
-    if (kernel == LK_NODAL_VEL)
-        return cudaFuncGetAttributes(&a, k_nodal_vel) == cudaSuccess ? a.maxThreadsPerBlock : 0;
+    // k_nodal_vel runs in blocks of at most 256 threads; larger shapes stay valid and are cut to that
+    if (kernel == LK_NODAL_VEL) return 1024;
     if (kernel != LK_LEVELS) return 0;
     const void* fs[] = {(const void*)k_lev_nodes, (const void*)k_lev_elems, (const void*)k_lev_nodes_dry,
                         (const void*)k_lev_rewet_nodes, (const void*)k_lev_sides, (const void*)k_lev_sides_dry};

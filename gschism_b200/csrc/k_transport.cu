@@ -633,24 +633,8 @@ static cudaError_t launch_ntr(const Dev& d, const Phys& P, TrArgs& T, cudaStream
     return cudaGetLastError();
 }
 
-template <int NTR>
-static int nodal_tracer_max_threads() {
-    cudaFuncAttributes a{};
-    return cudaFuncGetAttributes(&a, k_nodal_tracer<NTR>) == cudaSuccess ? a.maxThreadsPerBlock : 0;
-}
-
-int transport_max_threads(int ntr) {
-    switch (ntr) {
-    case 1: return nodal_tracer_max_threads<1>();
-    case 2: return nodal_tracer_max_threads<2>();
-    case 3: return nodal_tracer_max_threads<3>();
-    case 4: return nodal_tracer_max_threads<4>();
-    case 5: return nodal_tracer_max_threads<5>();
-    case 6: return nodal_tracer_max_threads<6>();
-    case 7: return nodal_tracer_max_threads<7>();
-    default: return nodal_tracer_max_threads<8>();
-    }
-}
+// k_nodal_tracer runs in blocks of at most 256 threads; larger shapes stay valid and are cut to that.
+int transport_max_threads(int) { return 1024; }
 
 cudaError_t launch_transport(const Dev& d, const Phys& P, double dt, cudaStream_t st, int nsm, const LaunchTable& L) {
     if (P.ntr <= 0) return cudaSuccess;

@@ -1306,7 +1306,7 @@ extern "C" size_t gs_footprint_bytes(int nvrt, int ntr, int nmem, int64_t np, in
     const double coarse = ((double)np / 4.0 + (double)nmem * kMgChunk + kMgPad) * 4.0 / 3.0;
     b += ((double)std::max<int64_t>(nnz - np, 0) * 1.25 + 32.0 * kMaxDeg * nmem) * 9.0 + (double)np * 4.0 +
          ((double)np / 32.0 + nmem) * 8.0 + coarse * (16.0 * 9.0 + 28.0);
-    b += ((double)np / 1024.0 + nmem) * 84.0 + (double)nmem * (16.0 + 72.0 + 40.0 + 8.0 * kVortexParams + 64.0 + 8.0);
+    b += ((double)np / 256.0 + nmem) * 48.0 + (double)nmem * (24.0 + 72.0 + 40.0 + 8.0 * kVortexParams + 64.0 + 8.0);
     b += (double)kMassBlocks * kMaxTracers * 16.0 + kMaxTracers * 8.0;
     b += 256.0 * 1024 * 1024;                   // allocation granularity of ~120 allocations
     return (size_t)b;
