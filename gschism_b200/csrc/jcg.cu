@@ -46,13 +46,14 @@ cudaError_t jcg_work_alloc(JcgWork*& w, const std::vector<int>& row0, const std:
     A((void**)&w->tile_part, 8 * (size_t)kPartialKinds * T);
     A((void**)&w->mem_atol2, 8 * nm);
     A((void**)&w->mem_ab, 64 * nm);
-    A((void**)&w->mctl, 4 * (6 * nm + 3));
+    A((void**)&w->mctl, 4 * (6 * nm + 4));
     if (e != cudaSuccess) return e;
     w->mdone = w->mctl; w->mouter = w->mctl + nm; w->minner = w->mctl + 2 * nm; w->mret = w->mctl + 3 * nm;
     w->mgen = w->mctl + 4 * nm; w->mcnt = (unsigned*)(w->mctl + 5 * nm);
     w->ndone = (unsigned*)(w->mctl + 6 * nm);
     w->status = w->mctl + 6 * nm + 1;
     w->bar = (unsigned*)(w->mctl + 6 * nm + 2);
+    w->nlev = (unsigned*)(w->mctl + 6 * nm + 3);
     // uploads on the caller's stream, never the legacy default stream (pageable sources are
     // staged before each call returns)
     cudaMemcpyAsync(w->mem_t0, mt0.data(), 4 * nm, cudaMemcpyHostToDevice, st);
@@ -61,7 +62,7 @@ cudaError_t jcg_work_alloc(JcgWork*& w, const std::vector<int>& row0, const std:
     cudaMemcpyAsync(w->mem_tr, mtr.data(), 4 * nm, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(w->tile_part, 0, 8 * (size_t)kPartialKinds * T, st);
     cudaMemsetAsync(w->mem_ab, 0, 64 * nm, st);
-    cudaMemsetAsync(w->mctl, 0, 4 * (6 * nm + 3), st);
+    cudaMemsetAsync(w->mctl, 0, 4 * (6 * nm + 4), st);
     cudaStreamSynchronize(st);
     return cudaGetLastError();
 }
@@ -76,7 +77,7 @@ void jcg_work_free(JcgWork* w) {
 cudaError_t jcg_clear(JcgWork* w, cudaStream_t st) {
     const size_t nm = w->nmem;
     cudaError_t e = cudaMemsetAsync(w->mdone, 0xFF, 4 * nm, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(w->mouter, 0, 4 * (5 * nm + 3), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w->mouter, 0, 4 * (5 * nm + 4), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(w->mgen, 0x7F, 4 * nm, st);
     return e;
 }

@@ -15,12 +15,13 @@ struct JcgWork {
     int32_t *mem_t0 = nullptr, *mem_row0 = nullptr, *mem_rows = nullptr, *mem_tr = nullptr;
     double *tile_part = nullptr, *mem_atol2 = nullptr, *mem_ab = nullptr;
     // per-member control words in one array: mdone, mouter, minner, mret, mgen, mcnt ([nmem] each),
-    // ndone, status (ERR_JCG_NOT_CONVERGED of the last solve), bar (grid barrier)
+    // ndone, status (ERR_JCG_NOT_CONVERGED of the last solve), bar (grid barrier), nlev (members
+    // iterating with the coarse correction)
     int32_t* mctl = nullptr;
     int32_t* status = nullptr;
     int32_t *mdone = nullptr, *mouter = nullptr, *minner = nullptr, *mret = nullptr, *mgen = nullptr;
     unsigned* mcnt = nullptr;
-    unsigned *ndone = nullptr, *bar = nullptr;
+    unsigned *ndone = nullptr, *bar = nullptr, *nlev = nullptr;
 };
 
 // Control words at the start of a solve: mdone = -1, mgen = 0x7f7f7f7f, the others 0.

@@ -99,3 +99,60 @@ def test_fp64_member_in_a_batch_beyond_shared_memory(native):
     assert mix.stats(0)["jcg_iters"] == solo.stats(0)["jcg_iters"]
     mix.close()
     solo.close()
+
+
+def _solve_ms(model, first, solves=8):
+    """Shortest time of the SOLVE phase over some steps (CUDA events)."""
+    import torch
+    from gschism_b200.autotune import PhaseTimer
+    timer = PhaseTimer(model, first_step=first)
+    ts = [timer.step()["SOLVE"] for _ in range(solves)]
+    torch.cuda.synchronize()
+    return min(ts)
+
+
+def test_batch_is_no_slower_than_its_members_one_after_another(native):
+    """A small member's iterations do not carry a large member's phases: one solve of the batch takes less
+    time than solves of its members in turn."""
+    from gschism_b200.model import Model
+    cs = [_basin(41, 40), _basin(42, 63), _basin(43, 200)]
+    times = []
+    for group in [cs] + [[c] for c in cs]:
+        m = Model(group, precision="fp32_ir")
+        m.step(8)
+        times.append(_solve_ms(m, 9))
+        m.close()
+    assert times[0] <= sum(times[1:]), times
+
+
+@pytest.mark.parametrize("side", [31, 32, 33])
+def test_elevation_at_the_line(native, oracle_lib, side):
+    """Both sides of the 1,024-row line between plain Jacobi and the hierarchy, against the oracle."""
+    from gschism_b200.model import Model
+    from oracle.step_api import OracleModel
+    c = _basin(50 + side, side)
+    o = OracleModel(c)
+    o.run(3)
+    g = Model([c], precision="fp32_ir")
+    g.step(3)
+    assert g.stats(0)["error_flags"] == 0
+    assert relerr(g.get(0, "ETA2"), o.get("ETA2")) <= 1e-9
+    g.close()
+
+
+@pytest.mark.parametrize("inner_maxiter", [1, 2, 400])
+def test_small_and_large_members_equal_their_solo_runs(native, inner_maxiter):
+    """Members on both sides of the line in one context, bit for bit their solo results; with one or two
+    iterations a sweep every member leaves the hierarchy after sweeps that do not halve the residual."""
+    from gschism_b200.model import Model
+    cs = [_basin(61, 20), _basin(62, 31), _basin(63, 32), _basin(64, 90)]
+    mix = Model(cs, precision="fp32_ir", ir_inner_maxiter=inner_maxiter)
+    mix.step(2)
+    for k, c in enumerate(cs):
+        solo = Model([c], precision="fp32_ir", ir_inner_maxiter=inner_maxiter)
+        solo.step(2)
+        assert np.array_equal(mix.get(k, "ETA2"), solo.get(0, "ETA2")), k
+        assert mix.stats(k)["jcg_iters"] == solo.stats(0)["jcg_iters"]
+        assert mix.stats(k)["jcg_outer"] == solo.stats(0)["jcg_outer"]
+        solo.close()
+    mix.close()

@@ -1,0 +1,70 @@
+"""Structure of the refinement solve's hierarchy (mg_setup.cpp) on the CPU: which members of a batch
+get one.  The choice depends on the member alone, so that a member gives the same bits alone and in
+any batch."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "gschism_b200", "csrc")
+
+HARNESS = r"""
+#include "mg.h"
+// mem_c of every member (its first row on level 1, -1: no hierarchy); returns -1 where mg_build refuses
+extern "C" int mg_members(int nmem, const int* rows, const int32_t* nnp_s, const int32_t* nnp, int32_t* mem_c) {
+    std::vector<int> row0(nmem), rw(rows, rows + nmem);
+    int n = 0;
+    for (int m = 0; m < nmem; m++) { row0[m] = n; n += rw[m]; }
+    std::vector<int32_t> s(nnp_s, nnp_s + n + 1), c(nnp, nnp + nnp_s[n]);
+    gs::MgHost H;
+    if (!gs::mg_build(row0, rw, s, c, true, H)) return -1;
+    for (int m = 0; m < nmem; m++) mem_c[m] = H.mem_c[m];
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def mg(tmp_path_factory):
+    d = tmp_path_factory.mktemp("mg")
+    src, lib = d / "harness.cpp", d / "libmg.so"
+    src.write_text(HARNESS)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-I/usr/local/cuda/include", str(src),
+                    os.path.join(CSRC, "mg_setup.cpp"), "-o", str(lib)], check=True)
+    return ctypes.CDLL(str(lib))
+
+
+def _lattice(nx, ny):
+    """Neighbour lists of a lattice with one diagonal (six neighbours inside)."""
+    out = []
+    for j in range(ny):
+        for i in range(nx):
+            out.append([(j + b) * nx + i + a for a, b in ((-1, 0), (1, 0), (0, -1), (0, 1), (1, 1), (-1, -1))
+                        if 0 <= i + a < nx and 0 <= j + b < ny])
+    return out
+
+
+def _members(mg, graphs):
+    rows = np.array([len(g) for g in graphs], dtype=np.int32)
+    flat, ptr, r0 = [], [0], 0
+    for g in graphs:
+        for nb in g:
+            flat.extend(r0 + c for c in nb)
+            ptr.append(len(flat))
+        r0 += len(g)
+    a = [np.array(v, dtype=np.int32) for v in (ptr, flat)]
+    mem_c = np.full(len(graphs), -7, dtype=np.int32)
+    p = [v.ctypes.data_as(ctypes.c_void_p) for v in (rows, a[0], a[1], mem_c)]
+    assert mg.mg_members(len(graphs), *p) == 0
+    return mem_c
+
+
+@pytest.mark.parametrize("nx,ny,on", [(20, 20, False), (31, 33, False), (32, 32, True), (50, 50, True), (63, 63, True)])
+def test_line_between_plain_and_hierarchy(mg, nx, ny, on):
+    """1,023 rows and fewer iterate without the hierarchy, alone and beside a large member."""
+    g, big = _lattice(nx, ny), _lattice(70, 70)
+    assert (_members(mg, [g])[0] >= 0) == on
+    c = _members(mg, [g, big])
+    assert (c[0] >= 0) == on and c[1] >= 0
