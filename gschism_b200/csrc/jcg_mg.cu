@@ -77,7 +77,8 @@ __device__ __forceinline__ void mg_share(const MgView& J, int sweep, Share& S, P
 }
 
 // Matrix entries pass through the SM once per product: they are read around the L1, which then
-// keeps the gathered vectors.
+// keeps the gathered vectors.  The structure is constant; the coarse levels' values are written earlier
+// in the same launch by other SMs, so values are never read through the non-coherent path.
 __device__ __forceinline__ int32_t ld_stream(const int32_t* p) {
     int32_t v;
     asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
@@ -85,7 +86,7 @@ __device__ __forceinline__ int32_t ld_stream(const int32_t* p) {
 }
 __device__ __forceinline__ float ld_stream(const float* p) {
     float v;
-    asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 

@@ -3,6 +3,7 @@ get one.  The choice depends on the member alone, so that a member gives the sam
 any batch."""
 import ctypes
 import os
+import re
 import subprocess
 
 import numpy as np
@@ -68,3 +69,12 @@ def test_line_between_plain_and_hierarchy(mg, nx, ny, on):
     assert (_members(mg, [g])[0] >= 0) == on
     c = _members(mg, [g, big])
     assert (c[0] >= 0) == on and c[1] >= 0
+
+
+def test_values_written_in_the_launch_are_read_coherently():
+    """The coarse matrices are written by the launch that reads them: ld.global.nc and __ldg, which need
+    data that no thread writes during the kernel, may only read the structure and the constant inputs."""
+    text = open(os.path.join(CSRC, "jcg_mg.cu")).read()
+    assert re.findall(r"ld\.global\.nc\S*\.(\w+) ", text) == ["s32"]
+    for arg in re.findall(r"__ldg\(([^;]*?)\)[;,]? ?", text):
+        assert not re.search(r"\.val\b|\bDinv\b|\.D\b|\.rh\b|\.e\b|\bJ\.[uzwpsdx]\b", arg), arg
