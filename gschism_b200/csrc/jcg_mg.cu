@@ -123,6 +123,8 @@ __device__ __forceinline__ void ring_request(Ring& R, int q, const MgMatrix& A, 
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+__device__ __forceinline__ void ring_drain() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
 // The warp's walk over a phase's slices: at(n) is the header of its n-th one.
 template <typename At>
 __device__ __forceinline__ void ring_open(Ring& R, const MgMatrix& A, At at) {
@@ -130,7 +132,7 @@ __device__ __forceinline__ void ring_open(Ring& R, const MgMatrix& A, At at) {
 #pragma unroll
     for (int q = 0; q < kDepth; q++) h[q] = at(q);
     // (copies of a walk that was opened and not run)
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    ring_drain();
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < kDepth; q++) ring_request(R, q, A, h[q]);
@@ -426,7 +428,8 @@ __device__ __forceinline__ RowVec row_vec(const MgView& J, const Part& q, int i)
     return {q.lev ? J.z[i] : J.u[i], J.w[i], J.p[i], J.s[i], J.d[i], J.u[i], __ldcg(J.diag + i)};
 }
 
-#define MG_SYNC() do { if (!bar.sync(J, stall)) return; } while (0)
+// (no thread leaves the kernel with copies of its own in flight)
+#define MG_SYNC() do { if (!bar.sync(J, stall)) { ring_drain(); return; } } while (0)
 
 __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
     __shared__ double sh[3][kT / 32];
@@ -674,6 +677,7 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
         }
         MG_SYNC();
     }
+    ring_drain();
     for (int m = blockIdx.x * kT + tid; m < nmem; m += gridDim.x * kT)
         if (*((volatile int32_t*)&J.mdone[m]) < 0) {
             J.mdone[m] = J.minner[m];

@@ -78,3 +78,15 @@ def test_values_written_in_the_launch_are_read_coherently():
     assert re.findall(r"ld\.global\.nc\S*\.(\w+) ", text) == ["s32"]
     for arg in re.findall(r"__ldg\(([^;]*?)\)[;,]? ?", text):
         assert not re.search(r"\.val\b|\bDinv\b|\.D\b|\.rh\b|\.e\b|\bJ\.[uzwpsdx]\b", arg), arg
+
+
+def test_no_exit_with_copies_in_flight():
+    """Every way out of the solve's kernel waits for the thread's own asynchronous copies first: slices are
+    requested before the barrier that may end the kernel."""
+    text = open(os.path.join(CSRC, "jcg_mg.cu")).read()
+    body = text[text.index("__global__"):text.index("static size_t mg_shared")]
+    sync = re.search(r"#define MG_SYNC\(\) (.*)", text).group(1)
+    assert re.search(r"ring_drain\(\);\s*return", sync)
+    assert "return;" not in body                       # the macro is the only early exit
+    loop = body[body.index("for (int sweep"):]
+    assert "ring_drain();" in loop[loop.rindex("MG_SYNC"):]
