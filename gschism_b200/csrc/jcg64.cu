@@ -335,14 +335,10 @@ struct Shape64 {
     size_t shared;
 };
 static cudaError_t jcg64_shape(bool sell, long long rows, int ntiles, int nmem, int nsm, Shape64& S) {
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     S.fn = sell ? (const void*)k_jcg64<true, true> : (const void*)k_jcg64<false, true>;
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, S.fn);
+    long long room = 0;
+    cudaError_t e = grant_shared(S.fn, room);
     if (e != cudaSuccess) return e;
-    const long long room = (long long)optin - (long long)fa.sharedSizeBytes;
     S.grid = std::max(1, std::min(ntiles, nsm));
     long long parts = (long long)(sizeof(Part) * share_parts(nmem, S.grid));
     if (parts > room) return cudaErrorInvalidConfiguration;
@@ -354,13 +350,14 @@ static cudaError_t jcg64_shape(bool sell, long long rows, int ntiles, int nmem, 
         const int grid = std::max(1, std::min(ntiles, 2 * nsm));
         const size_t shared = sizeof(Part) * share_parts(nmem, grid);
         int fit = 0;
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(shared, (size_t)4096));
+        long long room2 = 0;
+        e = grant_shared(fn, room2);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kT, shared);
         if (e != cudaSuccess) return e;
         if (fit >= 2) { S.fn = fn; S.grid = grid; S.entries = 0; S.shared = shared; return cudaSuccess; }
         S.shared = (size_t)parts + 12 * (size_t)S.entries;
     }
-    return cudaFuncSetAttribute(S.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.shared);
+    return cudaSuccess;
 }
 
 cudaError_t jcg64_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st, int nsm) {

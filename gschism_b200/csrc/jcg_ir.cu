@@ -273,26 +273,22 @@ cudaError_t jcg_ir_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st, int nsm
     J.check_every = a.check_every > 0 ? a.check_every : 1;
     // a row of a triangular mesh has about seven entries: the matrix is held when that many fit (a block
     // whose rows turn out to have more reads them from global memory)
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const void* fn = (const void*)k_jcg_ir<true>;
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    long long room = 0;
+    cudaError_t e = grant_shared(fn, room);
     if (e != cudaSuccess) return e;
     int grid = std::max(1, std::min(w->ntiles, nsm));
     J.max_parts = share_parts(1, grid);
     size_t shared = sizeof(Part) * J.max_parts;
-    J.cache_entries = (int)((optin - (long long)fa.sharedSizeBytes - (long long)shared) / 8);
+    J.cache_entries = (int)((room - (long long)shared) / 8);
     if (7LL * a.n <= (long long)J.cache_entries * grid) {
         shared += 8 * (size_t)J.cache_entries;
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
     } else {
         fn = (const void*)k_jcg_ir<false>;
         grid = std::max(1, std::min(w->ntiles, 2 * nsm));
         J.cache_entries = 0;
     }
-    if (e == cudaSuccess) e = jcg_clear(w, st);
+    e = jcg_clear(w, st);
     if (e != cudaSuccess) return e;
     void* args[] = {&J};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kT), args, shared, st);

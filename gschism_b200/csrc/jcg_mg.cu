@@ -693,12 +693,8 @@ static size_t mg_shared(int nmem, int grid) {
 
 // Two blocks per SM; one where the parts of very many members leave no room for two.
 static int mg_grid(int ntiles, int nmem, int nsm) {
-    int optin = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, k_jcg_mg);
-    cudaFuncSetAttribute(k_jcg_mg, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+    long long room = 0;
+    grant_shared((const void*)k_jcg_mg, room);
     const int grid = std::max(1, std::min(ntiles, 2 * nsm));
     int fit = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_jcg_mg, kT, mg_shared(nmem, grid));

@@ -282,4 +282,18 @@ __device__ __forceinline__ int tiles_of(const Part& q) { return (q.rows + q.tr -
 // (rows + extra members) / grid, each counting at least extra = rows / (8 grid), and two at its ends.
 inline int share_parts(int nmem, int grid) { return 12 + nmem / grid; }
 
+// Dynamic shared memory that a block of fn can have: all that the device grants beside fn's static part.
+// The limit is a property of the function on the device, shared by every context and host thread, so it is
+// always set to this one value; a launch asks for what it needs.
+inline cudaError_t grant_shared(const void* fn, long long& room) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    room = (long long)optin - (long long)fa.sharedSizeBytes;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
+}
+
 }  // namespace gs

@@ -78,3 +78,44 @@ def test_jcg_csr_mixed_precision(native, system):
     s.solve(rtol=1e-12, maxiter=1500, checkEvery=10)
     assert s.checkSolution() <= 1e-11
     s.close()
+
+
+def _tridiagonal(n):
+    """CSR of a diagonally dominant tridiagonal matrix."""
+    r = np.repeat(np.arange(n), 3)
+    c = r + np.tile([-1, 0, 1], n)
+    keep = (c >= 0) & (c < n)
+    r, c = r[keep], c[keep]
+    ptr = np.zeros(n + 1, dtype=np.int32)
+    ptr[1:] = np.cumsum(np.bincount(r, minlength=n))
+    return ptr, c.astype(np.int32), np.where(r == c, 2.5, -1.0)
+
+
+def test_solvers_of_two_threads_do_not_disturb_each_other(native):
+    """Solvers whose launches need different amounts of shared memory (one block, and several), solving at
+    the same time from two host threads: a kernel's limit is shared by both."""
+    import threading
+    from gschism_b200.solver import PCGSolverMultiGPU
+    rng = np.random.default_rng(5)
+    solvers, results = [], [None, None]
+    for n in (100, 3000):
+        A = _tridiagonal(n)
+        s = PCGSolverMultiGPU(None, [n], [A[2].size])
+        _fill(s, A, rng.standard_normal(n))
+        solvers.append(s)
+
+    def work(k):
+        try:
+            results[k] = [solvers[k].solve(rtol=1e-10, maxiter=200, checkEvery=5) for _ in range(1500)]
+        except Exception as e:       # reported by the main thread
+            results[k] = e
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for k, s in enumerate(solvers):
+        assert isinstance(results[k], list), results[k]
+        assert s.checkSolution() <= 1e-9
+        s.close()
