@@ -197,6 +197,9 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
         }
     }
     SYNC64();
+    // whether the block's first part still iterates, a copy of every thread's own: Part::on is cleared by one
+    // thread in phase A and read by the others only behind a barrier
+    bool first_on = S.n > 0 && part[0].on;
     for (int it = 0;; it++) {
         const double* pc = (it & 1) ? J.p1 : J.p0;
         double* pn = (it & 1) ? J.p0 : J.p1;
@@ -222,6 +225,7 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
             // the test of iteration it - 1
             const bool conv = it > 0 && (it % J.check_every == 0 || it == J.maxiter) && v[0] <= q.target;
             const bool done = conv || it == J.maxiter;
+            if (k == 0 && done) first_on = false;
             if (tid == 0) {
                 if (done) {
                     q.on = 0;
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
         // are loaded before the barrier
         double fx[kEarly], fr[kEarly], fq[kEarly], fp[kEarly], fd[kEarly];
         int fs = -1;
-        if (HELD && S.n > 0 && part[0].on) {
+        if (HELD && first_on) {
             const Part& q = part[0];
             const int per = q.tr / 32, last = min(q.e * per, (q.rows + 31) / 32);
             fs = q.a * per + ((w - q.a * per) & (kT / 32 - 1));
