@@ -52,14 +52,15 @@ struct MgHost {
     std::vector<int32_t> mem_s, mem_c, chunk_mem, row_at;
     std::vector<int2> chunk_fine;
 };
-// Members with fewer rows use plain Jacobi (no hierarchy).  A solve alone, plain and with the hierarchy:
+// Members with fewer rows iterate with plain Jacobi (no hierarchy).  A solve alone, plain and with the hierarchy:
 // 400 rows 0.93 and 1.42 ms, 784 rows 1.22 and 1.27, 961 rows 1.48 and 1.46, 1,225 rows 1.67 and 1.37, 3,969
 // rows 2.96 and 1.92; beside a 40,000-row member 961 rows take 3.4 and 2.3 ms, 3,969 rows 6.8 and 2.4.
 constexpr int kMgMinRows = 1024;
 // nnp_s/nnp: node -> nodes of the batch (global rows, ball order); row0/rows per member.
-// Returns false when a matrix needs more than 32-bit offsets or a coarse row has more neighbours
-// than a map byte can name; without `levels` no member gets a hierarchy.
+// A member has a hierarchy from kMgMinRows rows on, unless one of its coarse rows has more neighbours than
+// a map byte can name: a property of the member alone.  Returns false when a matrix needs more than 32-bit
+// offsets.
 bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const std::vector<int32_t>& nnp_s,
-              const std::vector<int32_t>& nnp, bool levels, MgHost& H);
+              const std::vector<int32_t>& nnp, MgHost& H);
 
 }  // namespace gs

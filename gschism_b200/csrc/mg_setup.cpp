@@ -16,10 +16,13 @@ struct Graph {
     std::vector<int32_t> ptr, cols;
 };
 
-}  // namespace
+// What build() found: everything built, offsets beyond 32 bits, or (>= 0) the member with a coarse row
+// wider than a map byte can name.
+enum { kBuilt = -1, kTooLarge = -2 };
 
-bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const std::vector<int32_t>& nnp_s,
-              const std::vector<int32_t>& nnp, bool levels, MgHost& H) {
+// `on`: members with a hierarchy
+int build(const std::vector<int>& row0, const std::vector<int>& rows, const std::vector<int32_t>& nnp_s,
+          const std::vector<int32_t>& nnp, const std::vector<uint8_t>& on, MgHost& H) {
     H = MgHost();
     const int nmem = (int)rows.size();
     // fine slices, relative to each member's first row
@@ -37,7 +40,7 @@ bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const 
             off += 32LL * w;
         }
     }
-    if (off > 0x7fffffffLL) return false;
+    if (off > 0x7fffffffLL) return kTooLarge;
     H.A.idx.resize((size_t)off);
     H.A.map.assign((size_t)off, kMgDiag);
     for (int m = 0; m < nmem; m++)
@@ -56,7 +59,7 @@ bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const 
     // share one parent and a member's first row has a whole number of ancestors
     int n1 = 0;
     for (int m = 0; m < nmem; m++) {
-        if (!levels || rows[m] < kMgMinRows) continue;
+        if (!on[m]) continue;
         H.mem_c[m] = n1;
         const int c = ((rows[m] + 3) / 4 + kMgChunk - 1) / kMgChunk;
         n1 += c * kMgChunk;
@@ -85,7 +88,7 @@ bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const 
                     if (J == I) continue;
                     const size_t slot = std::find(own.begin(), own.end(), J) - own.begin();
                     if (slot == own.size()) own.push_back(J);
-                    if (slot >= (size_t)kMgMaxSlots) return false;
+                    if (slot >= (size_t)kMgMaxSlots) return m;
                     H.A.map[(size_t)H.row_at[i] + 32 * (size_t)k] = (uint8_t)slot;
                 }
             }
@@ -105,7 +108,7 @@ bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const 
             A.sl[s] = int2{(int)off, w};
             off += 32LL * w;
         }
-        if (off > 0x7fffffffLL) return false;
+        if (off > 0x7fffffffLL) return kTooLarge;
         A.idx.resize((size_t)off);
         for (int s = 0; s < n / 32; s++)
             for (int l = 0; l < 32; l++) {
@@ -126,7 +129,7 @@ bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const 
                     if (J == I) continue;
                     const size_t slot = std::find(own.begin(), own.end(), J) - own.begin();
                     if (slot == own.size()) own.push_back(J);
-                    if (slot >= (size_t)kMgMaxSlots) return false;
+                    if (slot >= (size_t)kMgMaxSlots) return H.chunk_mem[((size_t)I << (2 * (lev + 1))) / kMgChunk];
                     A.map[(size_t)A.sl[i / 32].x + 32 * (size_t)k + i % 32] = (uint8_t)slot;
                 }
             c.cols.insert(c.cols.end(), own.begin(), own.end());
@@ -134,7 +137,21 @@ bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const 
         }
         g = std::move(c);
     }
-    return true;
+    return kBuilt;
+}
+
+}  // namespace
+
+bool mg_build(const std::vector<int>& row0, const std::vector<int>& rows, const std::vector<int32_t>& nnp_s,
+              const std::vector<int32_t>& nnp, MgHost& H) {
+    // a member with too wide a coarse row goes without the hierarchy, the others keep theirs
+    std::vector<uint8_t> on(rows.size());
+    for (size_t m = 0; m < rows.size(); m++) on[m] = rows[m] >= kMgMinRows;
+    for (;;) {
+        const int r = build(row0, rows, nnp_s, nnp, on, H);
+        if (r < 0) return r == kBuilt;
+        on[r] = 0;
+    }
 }
 
 }  // namespace gs

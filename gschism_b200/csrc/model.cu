@@ -500,7 +500,7 @@ static gs_status prepare_host(gs_ctx* c) {
     if (c->cfg.precision == GS_FP32_IR) {
         std::vector<int> row0, rows;
         for (auto& m : c->mem) { row0.push_back(m.np0); rows.push_back(m.np); }
-        if (!mg_build(row0, rows, B.nnp_s, B.nnp, true, pr->mg) && !mg_build(row0, rows, B.nnp_s, B.nnp, false, pr->mg))
+        if (!mg_build(row0, rows, B.nnp_s, B.nnp, pr->mg))
             return c->fail(GS_ERR_ARG, "elevation matrix too large for 32-bit offsets");
     }
     c->prep = guard.release();

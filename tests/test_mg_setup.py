@@ -20,7 +20,7 @@ extern "C" int mg_members(int nmem, const int* rows, const int32_t* nnp_s, const
     for (int m = 0; m < nmem; m++) { row0[m] = n; n += rw[m]; }
     std::vector<int32_t> s(nnp_s, nnp_s + n + 1), c(nnp, nnp + nnp_s[n]);
     gs::MgHost H;
-    if (!gs::mg_build(row0, rw, s, c, true, H)) return -1;
+    if (!gs::mg_build(row0, rw, s, c, H)) return -1;
     for (int m = 0; m < nmem; m++) mem_c[m] = H.mem_c[m];
     return 0;
 }
@@ -69,6 +69,40 @@ def test_line_between_plain_and_hierarchy(mg, nx, ny, on):
     assert (_members(mg, [g])[0] >= 0) == on
     c = _members(mg, [g, big])
     assert (c[0] >= 0) == on and c[1] >= 0
+
+
+def _hub(n, spokes):
+    """A path of n rows whose first row is also a neighbour of every eighth one, `spokes` times."""
+    g = [[j for j in (i - 1, i + 1) if 0 <= j < n] for i in range(n)]
+    for k in range(1, spokes + 1):
+        g[0].append(8 * k)
+        g[8 * k].append(0)
+    return g
+
+
+@pytest.mark.parametrize("spokes,on", [(200, True), (300, False)])
+def test_wide_coarse_row_drops_only_its_own_member(mg, spokes, on):
+    """A coarse row of more than 255 neighbours leaves that member without the hierarchy; its neighbours in
+    the batch keep theirs, as they would alone."""
+    hub, other = _hub(8 * 320, spokes), _lattice(40, 40)
+    assert (_members(mg, [hub])[0] >= 0) == on
+    for batch, k in (([other, hub, other], 1), ([hub, other], 0)):
+        c = _members(mg, batch)
+        assert (c[k] >= 0) == on
+        assert all(v >= 0 for i, v in enumerate(c) if i != k)
+
+
+def test_wide_row_on_a_higher_level(mg):
+    """300 neighbours of the sixteen rows of one level-2 aggregate, at most 80 of any four of them."""
+    n = 16 * 400
+    g = [[j for j in (i - 1, i + 1) if 0 <= j < n] for i in range(n)]
+    for k in range(300):
+        a, b = k % 16, 16 * (k + 10)
+        g[a].append(b)
+        g[b].append(a)
+    other = _lattice(40, 40)
+    c = _members(mg, [other, g, other])
+    assert c[0] >= 0 and c[1] < 0 and c[2] >= 0
 
 
 def test_values_written_in_the_launch_are_read_coherently():
