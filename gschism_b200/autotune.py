@@ -93,9 +93,11 @@ def tune_model(model, kernels: Sequence[str] = TUNE_ORDER, rounds: int = 3,
         for c in candidates(k):
             try:
                 model.set_launch(k, *c)
-                valid.append(c)
             except GsError:
                 continue
+            c = tuple(model.get_launch(k))      # the shape that runs
+            if c not in valid:
+                valid.append(c)
         if not valid:
             model.set_launch(k, *start)
             chosen[k] = start

@@ -58,6 +58,10 @@ enum : int {
     LK_NODAL_TRACER, LK_LEVELS, LK_COUNT
 };
 struct LaunchShape { int block, per_sm; };
+// The node gathers (nodal velocities, nodal tracers) are compiled for blocks of at most this many threads;
+// a larger shape is accepted and entered in the table as this one (gs_set_launch), so the table always
+// holds what runs.
+constexpr int kGatherThreads = 256;
 struct JcgTiling {
     int tiles = 296;        // tiles of a large member (two per SM)
     int min_rows = 256;     // smallest tile: a 30k-row member still reaches most SMs (mixed-precision solve

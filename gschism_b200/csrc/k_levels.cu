@@ -134,7 +134,7 @@ __global__ void k_lev_sides_dry(Dev d) {
 // a node, 235 with runs of 4; on 360k nodes 656 and 512, 489 with runs of 3, which cost 10% on 40k nodes.)
 constexpr int kNodeRun = 4;
 
-__global__ void __launch_bounds__(256) k_nodal_vel(Dev d, Phys P) {
+__global__ void __launch_bounds__(kGatherThreads) k_nodal_vel(Dev d, Phys P) {
     const int NP = d.NP, NE = d.NE, NS = d.NS, nvrt = P.nvrt, ka = blockIdx.y * kNodeRun;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NP; i += gridDim.x * blockDim.x) {
         const int q0 = d.nne_s[i], q1 = d.nne_s[i + 1];
@@ -227,13 +227,12 @@ void launch_levels(const Dev& d, const Phys& P, const VG& vg, int it, cudaStream
 
 void launch_nodal_vel(const Dev& d, const Phys& P, cudaStream_t st, int nsm, const LaunchTable& L) {
     const LaunchShape& s = L.k[LK_NODAL_VEL];
-    k_nodal_vel<<<dim3(grid_of(d.NP, s, nsm), (P.nvrt + kNodeRun - 1) / kNodeRun), std::min(s.block, 256), 0, st>>>(d, P);
+    k_nodal_vel<<<dim3(grid_of(d.NP, s, nsm), (P.nvrt + kNodeRun - 1) / kNodeRun), s.block, 0, st>>>(d, P);
 }
 
 int levels_max_threads(int kernel) {
     cudaFuncAttributes a{};
-    // k_nodal_vel runs in blocks of at most 256 threads; larger shapes stay valid and are cut to that
-    if (kernel == LK_NODAL_VEL) return 1024;
+    if (kernel == LK_NODAL_VEL) return 1024;       // entered as kGatherThreads at most
     if (kernel != LK_LEVELS) return 0;
     const void* fs[] = {(const void*)k_lev_nodes, (const void*)k_lev_elems, (const void*)k_lev_nodes_dry,
                         (const void*)k_lev_rewet_nodes, (const void*)k_lev_sides, (const void*)k_lev_sides_dry};

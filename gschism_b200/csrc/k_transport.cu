@@ -547,7 +547,7 @@ constexpr int nodal_run() { return NTR <= 2 ? 3 : (NTR <= 4 ? 3 : 2); }
 // elements in the same order as a node-by-node loop.  (160k nodes, 30 levels, 2 tracers: 239 us with one
 // level per thread, 167 with runs of 3, 174 with runs of 5.)
 template <int NTR>
-__global__ void __launch_bounds__(256) k_nodal_tracer(Dev d, Phys P) {
+__global__ void __launch_bounds__(kGatherThreads) k_nodal_tracer(Dev d, Phys P) {
     constexpr int R = nodal_run<NTR>();
     const int NP = d.NP, NE = d.NE, nvrt = P.nvrt, ivrt = nvrt - 1, ka = blockIdx.y * R;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NP; i += gridDim.x * blockDim.x) {
@@ -629,11 +629,11 @@ static cudaError_t launch_ntr(const Dev& d, const Phys& P, TrArgs& T, cudaStream
     else if (P.tvd) launch_vertical<NTR, true, false>(d, P, T.dt, st, nsm);
     else launch_vertical<NTR, false, false>(d, P, T.dt, st, nsm);
     k_nodal_tracer<NTR><<<dim3(grid_of(d.NP, nt, nsm), (P.nvrt + nodal_run<NTR>() - 1) / nodal_run<NTR>()),
-                          std::min(nt.block, 256), 0, st>>>(d, P);
+                          nt.block, 0, st>>>(d, P);
     return cudaGetLastError();
 }
 
-// k_nodal_tracer runs in blocks of at most 256 threads; larger shapes stay valid and are cut to that.
+// k_nodal_tracer (shapes above kGatherThreads are entered as that)
 int transport_max_threads(int) { return 1024; }
 
 cudaError_t launch_transport(const Dev& d, const Phys& P, double dt, cudaStream_t st, int nsm, const LaunchTable& L) {

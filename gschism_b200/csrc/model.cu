@@ -876,7 +876,8 @@ gs_status gs_set_launch(gs_ctx* c, int kernel, int a, int b) {
     } else {
         const int mx = max_threads_of(kernel, c->cfg.ntr);
         if (a < 32 || a % 32 != 0 || a > mx || b < 1 || b > 64) return GS_ERR_ARG;
-        c->launch.k[kernel] = LaunchShape{a, b};
+        const bool gather = kernel == LK_NODAL_VEL || kernel == LK_NODAL_TRACER;
+        c->launch.k[kernel] = LaunchShape{gather ? std::min(a, kGatherThreads) : a, b};
     }
     // the captured step holds the old shapes
     if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }

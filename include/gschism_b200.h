@@ -231,6 +231,8 @@ gs_status gs_get_stats(gs_ctx* ctx, int member, gs_stats* out);
    launch shapes are fixed in its kernel wrappers).  For the stream kernels a = threads per block
    (a multiple of 32, at most what the compiled kernel allows) and b = the grid cap in blocks per
    SM (1..64); the kernels stride over their entities, so results do not depend on the shape.
+   GS_K_NODAL_VEL and GS_K_NODAL_TRACER take up to 1024 threads and run with 256 at most;
+   gs_get_launch reports the shape that runs.
    GS_K_JCG_TILES: a = tiles a large member is cut into, b = the smallest tile in rows (a
    multiple of 32); this changes the order of the solver's partial sums.  A change takes effect
    at the next launch (the captured step is recaptured). */

@@ -59,3 +59,23 @@ def test_cache_key_size_class():
     c = cases.channel()
     k = autotune.cache_key([c], "fp64", "B200")
     assert k.startswith("B200|fp64|nvrt=10|ntr=1|itr_met=1|nodes~2^11")
+
+
+class CuttingModel(FakeModel):
+    """A library that runs the node gathers with 256 threads at most and reports that."""
+
+    def set_launch(self, k, a, b):
+        super().set_launch(k, min(a, 256) if k in ("NODAL_VEL", "NODAL_TRACER") else a, b)
+
+
+def test_tuner_times_and_reports_the_shapes_that_run():
+    m = CuttingModel()
+    seen = []
+
+    def measure():
+        seen.append(m.get_launch("NODAL_VEL"))
+        return dict(m.measure(), NODAL_VEL=1.0 / m.get_launch("NODAL_VEL")[0])
+
+    got = autotune.tune_model(m, kernels=["NODAL_VEL"], rounds=1, measure=measure)
+    assert len(seen) == len(set(seen))              # each shape that runs is timed once
+    assert got["NODAL_VEL"][0] == 256 and got["NODAL_VEL"] == m.get_launch("NODAL_VEL")

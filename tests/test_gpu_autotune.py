@@ -42,3 +42,24 @@ def test_invalid_shapes_rejected(native):
         with pytest.raises(GsError):
             m.set_launch(k, a, b)
     assert m.get_launch("BTRACK") == (128, 32)
+
+
+def test_reported_shape_is_the_one_that_runs(native):
+    """The node gathers take shapes of up to 1,024 threads and run with 256 at most; gs_get_launch says so,
+    and the results do not depend on it."""
+    from gschism_b200.model import Model
+    c = cases.channel()
+    ref, m = Model([c]), Model([c])
+    for k in ("NODAL_VEL", "NODAL_TRACER"):
+        for block in (512, 1024):
+            m.set_launch(k, block, 8)
+            assert m.get_launch(k) == (256, 8)
+        m.set_launch(k, 64, 8)
+        assert m.get_launch(k) == (64, 8)
+        m.set_launch(k, 512, 1)
+    ref.step(3)
+    m.step(3)
+    for f in ("NODE_U2", "NODE_W2", "NODE_TR"):
+        assert np.array_equal(m.get(0, f), ref.get(0, f)), f
+    ref.close()
+    m.close()
