@@ -14,11 +14,15 @@ iteration), and moves to the next kernel.
     autotune.apply(model, shapes)
 
 Results are cached in a JSON file (``GSCHISM_TUNE_CACHE`` or ``_build/tune_cache.json`` next to
-the library) keyed by the GPU, the precision, the vertical grid, the tracer count and the size
-class (log2 of the node count), so a serving loop tunes a size class once.
+the library) keyed by the GPU, the precision, the vertical grid, the tracer count, the size
+class (log2 of the node count) and the kernels' sources, so a serving loop tunes a size class once
+and a plan timed on other kernels is not used.
 """
 from __future__ import annotations
 
+import functools
+import glob
+import hashlib
 import json
 import math
 import os
@@ -130,13 +134,27 @@ def cache_path() -> str:
     return os.path.join(build.BUILD, "tune_cache.json")
 
 
+@functools.lru_cache(maxsize=None)
+def kernel_revision(src: Optional[str] = None) -> str:
+    """Short hash of the kernels' sources (of the library itself where they are not installed)."""
+    from . import build
+    src = src or build.SRC
+    files = sorted(f for f in glob.glob(os.path.join(src, "*")) if f.endswith((".cu", ".cuh", ".h", ".cpp")))
+    h = hashlib.sha1()
+    for f in files or [build.LIB]:
+        h.update(os.path.basename(f).encode())
+        with open(f, "rb") as fh:
+            h.update(fh.read())
+    return h.hexdigest()[:12]
+
+
 def cache_key(cases, precision: str, gpu: str) -> str:
     c0 = cases[0]
     nodes = sum(int(c.n_nodes) for c in cases)
     cls = int(round(math.log2(max(nodes, 1))))
     p = c0.params
     return (f"{gpu}|{precision}|nvrt={c0.vgrid.nvrt}|ntr={c0.ntracers}|itr_met={p.itr_met}|"
-            f"nodes~2^{cls}")
+            f"nodes~2^{cls}|kernels={kernel_revision()}")
 
 
 def load_cache(path: Optional[str] = None) -> Dict[str, Dict[str, List[int]]]:

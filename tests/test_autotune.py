@@ -79,3 +79,14 @@ def test_tuner_times_and_reports_the_shapes_that_run():
     got = autotune.tune_model(m, kernels=["NODAL_VEL"], rounds=1, measure=measure)
     assert len(seen) == len(set(seen))              # each shape that runs is timed once
     assert got["NODAL_VEL"][0] == 256 and got["NODAL_VEL"] == m.get_launch("NODAL_VEL")
+
+
+def test_cache_key_names_the_kernels(tmp_path):
+    """A plan timed on other kernels is not found."""
+    from gschism_b200 import cases
+    a, b = tmp_path / "a", tmp_path / "b"
+    for d, body in ((a, "one"), (b, "two")):
+        d.mkdir()
+        (d / "k.cu").write_text(body)
+    assert autotune.kernel_revision(str(a)) != autotune.kernel_revision(str(b))
+    assert autotune.cache_key([cases.channel()], "fp64", "B200").endswith("|kernels=" + autotune.kernel_revision())
