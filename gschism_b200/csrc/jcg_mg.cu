@@ -9,7 +9,8 @@
 // coarse correction: z = w0 D^-1 r + c P V(P^T r), with P piecewise constant over four consecutive
 // rows (rows follow a Hilbert curve, so an aggregate is compact) and V one V(1,1) cycle with damped
 // Jacobi over kMgLevels levels of four-fold aggregation whose matrices are Galerkin sums.  Members
-// below kMgMinRows rows keep plain Jacobi (z = D^-1 r).
+// below kMgMinRows rows are solved apart (jcg_small.cu); a member whose coarse rows are too wide for the
+// hierarchy, or whose sweeps twice failed to halve the residual, iterates with plain Jacobi (z = D^-1 r).
 //
 // The preconditioner is symmetric positive definite for any weights because every smoother is
 // convergent: a row-scaled element matrix of a triangle is semi-definite with trace 3 (2 or 1 when an
@@ -559,9 +560,9 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
         }
         __syncthreads();
         // The cycle runs while a member iterates with it: members that iterate longer without it do not
-        // pay for its eight barriers (members of 900 to 40,000 rows: 3.9 ms a solve, 11.1 when every
-        // iteration walked through the cycle).  nstop and nlev are read behind a barrier after O2 or F2,
-        // which alone change them, so every block reads the same values.
+        // pay for its eight barriers (a plain iteration takes 7 to 10 us, one with the cycle 30 to 40).
+        // nstop and nlev are read behind a barrier after O2 or F2, which alone change them, so every block
+        // reads the same values.
         bool cycle = with_levels != 0;
         for (int it = 0; it <= J.inner_maxiter; it++) {
             if (cycle) {
@@ -723,7 +724,8 @@ cudaError_t jcg_mg_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st, int nsm
     J.max_parts = share_parts(w->nmem, grid);
     J.max_on = std::min(w->nmem, kFlags);
     cudaError_t e = jcg_clear(w, st);
-    if (e != cudaSuccess) return e;
+    if (e == cudaSuccess && w->nsmall > 0) e = jcg_small_launch(a, w, st);
+    if (e != cudaSuccess || w->nsmall == w->nmem) return e;
     int lev = a.mg->lv[0].n > 0 ? 1 : 0;
     void* args[] = {&J, &lev};
     return cudaLaunchCooperativeKernel((const void*)k_jcg_mg, dim3(grid), dim3(kT), args,

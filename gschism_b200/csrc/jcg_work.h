@@ -10,6 +10,7 @@ struct JcgArgs;
 
 struct JcgWork {
     int nmem = 0, ntiles = 0;
+    int nsmall = 0;                  // members below kMgMinRows rows
     bool sell = false;               // rows in the SELL-32 layout of a context, else a caller's CSR
     // per member: first tile, first row, rows, rows per tile
     int32_t *mem_t0 = nullptr, *mem_row0 = nullptr, *mem_rows = nullptr, *mem_tr = nullptr;
@@ -28,8 +29,9 @@ struct JcgWork {
 cudaError_t jcg_clear(JcgWork* w, cudaStream_t st);
 // jcg64.cu: the FP64 solve
 cudaError_t jcg64_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st, int nsm);
-// jcg_mg.cu: the refinement solve of a context (a.mg set)
+// jcg_mg.cu: the refinement solve of a context (a.mg set); jcg_small.cu: its members below kMgMinRows rows
 cudaError_t jcg_mg_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st, int nsm);
+cudaError_t jcg_small_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st);
 // jcg_ir.cu: the refinement solve of a caller's CSR matrix
 cudaError_t jcg_ir_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st, int nsm);
 

@@ -52,9 +52,10 @@ struct MgHost {
     std::vector<int32_t> mem_s, mem_c, chunk_mem, row_at;
     std::vector<int2> chunk_fine;
 };
-// Members with fewer rows iterate with plain Jacobi (no hierarchy).  A solve alone, plain and with the hierarchy:
-// 400 rows 0.93 and 1.42 ms, 784 rows 1.22 and 1.27, 961 rows 1.48 and 1.46, 1,225 rows 1.67 and 1.37, 3,969
-// rows 2.96 and 1.92; beside a 40,000-row member 961 rows take 3.4 and 2.3 ms, 3,969 rows 6.8 and 2.4.
+// Members with fewer rows have no hierarchy and are solved by one block each (jcg_small.cu).  961 rows: 0.37
+// ms alone, 1.46 with the hierarchy; 256 members of 900 rows 0.64 and 3.3 ms.  Beside a 40,000-row member the
+// block's time adds to the solve's (900 rows: 2.7 ms, 2.3 with the hierarchy), and more with every row, so
+// the line stays at the size that a block's threads hold two rows of.
 constexpr int kMgMinRows = 1024;
 // nnp_s/nnp: node -> nodes of the batch (global rows, ball order); row0/rows per member.
 // A member has a hierarchy from kMgMinRows rows on, unless one of its coarse rows has more neighbours than

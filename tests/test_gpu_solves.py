@@ -127,7 +127,7 @@ def test_batch_is_no_slower_than_its_members_one_after_another(native):
 
 @pytest.mark.parametrize("side", [31, 32, 33])
 def test_elevation_at_the_line(native, oracle_lib, side):
-    """Both sides of the 1,024-row line between plain Jacobi and the hierarchy, against the oracle."""
+    """Both sides of the 1,024-row line between a block's own solve and the hierarchy, against the oracle."""
     from gschism_b200.model import Model
     from oracle.step_api import OracleModel
     c = _basin(50 + side, side)
@@ -156,3 +156,79 @@ def test_small_and_large_members_equal_their_solo_runs(native, inner_maxiter):
         assert mix.stats(k)["jcg_outer"] == solo.stats(0)["jcg_outer"]
         solo.close()
     mix.close()
+
+
+@pytest.mark.parametrize("side", [6, 8, 22, 23])
+def test_elevation_of_a_block_member(native, oracle_lib, side):
+    """Members solved by one block: fewer rows than a warp's two slices, and both sides of one row per
+    thread, against the oracle."""
+    from gschism_b200.model import Model
+    from oracle.step_api import OracleModel
+    c = _basin(70 + side, side)
+    o = OracleModel(c)
+    o.run(3)
+    g = Model([c], precision="fp32_ir")
+    g.step(3)
+    assert g.stats(0)["error_flags"] == 0
+    assert relerr(g.get(0, "ETA2"), o.get("ETA2")) <= 1e-9
+    g.close()
+
+
+def test_parked_block_member_is_done_at_once(native):
+    """A zero right-hand side: solved by x = 0 without an iteration, beside members that iterate."""
+    from gschism_b200.model import Model
+    cs = [_basin(81, 20), _basin(82, 25), _basin(83, 40)]
+    m = Model(cs, precision="fp32_ir")
+    m.park(0, m.member_state(0))
+    m.step(2)
+    assert m.stats(0)["jcg_iters"] == 0 and m.stats(0)["error_flags"] == 0
+    assert np.abs(m.get(0, "ETA2")).max() == 0.0
+    for k in (1, 2):
+        solo = Model(cs[k:k + 1], precision="fp32_ir")
+        solo.step(2)
+        assert np.array_equal(m.get(k, "ETA2"), solo.get(0, "ETA2"))
+        solo.close()
+    m.close()
+
+
+def test_timed_out_block_member_is_reported_and_the_context_recovers(native):
+    """The recovery path (test_gpu_recovery.py) with a stalled member that one block solves, alone and beside
+    a large member: the wait runs out, is reported once, and the context steps on bit for bit."""
+    from gschism_b200 import _lib as L
+    from gschism_b200.model import Model
+    for cs in ([_basin(84, 20)], [_basin(84, 20), _basin(85, 50)]):
+        ref, m = (Model(cs, precision="fp32_ir") for _ in range(2))
+        ref.step(3)
+        m.step(2)
+        saved = [m.member_state(k) for k in range(len(cs))]
+        m.set_wait_limit(1 << 14)
+        m.test_stall_solve(0)
+        m.step(1)
+        with pytest.raises(L.GsError) as ei:
+            m.sync()
+        assert ei.value.status == L.GS_ERR_TIMEOUT
+        m.sync()
+        m.test_stall_solve(-1)
+        m.set_wait_limit(0)
+        for k in range(len(cs)):
+            m.put_member_state(k, saved[k])
+        m.phase("BEGIN", 2)
+        m.step(1)
+        m.sync()
+        for k in range(len(cs)):
+            assert np.array_equal(m.get(k, "ETA2"), ref.get(k, "ETA2")), k
+            assert m.stats(k)["error_flags"] == 0
+        m.close()
+        ref.close()
+
+
+def test_many_small_members_do_not_wait_for_one_another(native):
+    """256 members of 400 rows take less than three times the time of one."""
+    from gschism_b200.model import Model
+    times = []
+    for n in (1, 256):
+        m = Model([_basin(100 + k, 20) for k in range(n)], precision="fp32_ir")
+        m.step(8)
+        times.append(_solve_ms(m, 9))
+        m.close()
+    assert times[1] <= 3.0 * times[0], times
