@@ -103,6 +103,21 @@ __device__ __forceinline__ void row_products(const View64& J, const double* cv, 
     }
 }
 
+// f(part, totals of kinds [k0, k0 + NV)), by one thread, for every part of the block that still iterates.  A
+// warp adds a part's partials, so a block waits for one round trip, not for one per part.
+template <int NV, typename F>
+__device__ __forceinline__ void part_totals(const View64& J, const Share& S, Part* part, int k0, F f) {
+    __syncthreads();
+    for (int k = threadIdx.x >> 5; k < S.n; k += kT / 32) {
+        Part& q = part[k];
+        if (!q.on) continue;
+        double v[NV];
+        lane_totals<NV>(J, q.t0, tiles_of(q), k0, v);
+        if ((threadIdx.x & 31) == 0) f(q, v);
+    }
+    __syncthreads();
+}
+
 #define SYNC64() do { if (!bar.sync(J, stall)) return; } while (0)
 
 // partial kinds: a phase never writes the kinds it reads, since a slower block may not have read yet
@@ -112,9 +127,15 @@ enum { K_PQ = 0, K_RR = 1, K_RZ = 2 };
 // each scalar).  Otherwise, for a matrix larger than the chip's shared memory, two blocks per SM and
 // nothing ahead: such a solve is bound by the gathers in flight (1M rows: 55 us in the first form,
 // 39.7 in the second, 43.0 before).
-template <bool SELL, bool HELD>
+//
+// MANY: a batch whose blocks hold tiles of several members (more tiles than blocks).  A block takes the totals
+// of all its parts at once and no products ahead of them: 16 members of 8,100 rows 5.6 ms a solve, 6.3 part by
+// part; 64 members of 8,100 rows 8.9 and 9.5.  A block of one part keeps what it needs of it in registers over
+// the barriers, which that form does not (30k rows: 4.3 ms, 4.5 in it).
+template <bool SELL, bool HELD, bool MANY>
 __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
     constexpr int kEarly = 2;
+    constexpr bool kAhead = HELD && !MANY;   // products gathered before the totals are known
     __shared__ TileSums ts;
     __shared__ Share S;
     __shared__ double tot[3];
@@ -204,30 +225,11 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
         const double* pc = (it & 1) ? J.p1 : J.p0;
         double* pn = (it & 1) ? J.p0 : J.p1;
         // ---- A
-        for (int k = 0; k < S.n; k++) {
-            Part& q = part[k];
-            if (!q.on) continue;
-            const int per = q.tr / 32, first = q.a * per + ((w - q.a * per) & (kT / 32 - 1));
-            const int last = min(q.e * per, (q.rows + 31) / 32);
-            double az[kEarly], ap[kEarly], zi[kEarly], pi[kEarly];
-#pragma unroll
-            for (int j = 0; HELD && j < kEarly; j++) {
-                const int s = first + j * (kT / 32), o = 32 * s + lane, i = q.row0 + o;
-                az[j] = ap[j] = zi[j] = pi[j] = 0.0;
-                if (s < last && o < q.rows) {
-                    row_products<SELL, HELD, 2>(J, cv, ci, q.sl, i, J.z, pc, az[j], ap[j]);
-                    zi[j] = J.z[i]; pi[j] = pc[i];
-                }
-            }
-            const double rz_old = q.gp;
-            double v[2];
-            totals<2>(J, q.t0, tiles_of(q), K_RR, v, tot);
-            // the test of iteration it - 1
-            const bool conv = it > 0 && (it % J.check_every == 0 || it == J.maxiter) && v[0] <= q.target;
-            const bool done = conv || it == J.maxiter;
-            if (k == 0 && done) first_on = false;
-            if (tid == 0) {
-                if (done) {
+        if constexpr (MANY) {
+            part_totals<2>(J, S, part, K_RR, [&](Part& q, const double (&v)[2]) {
+                // the test of iteration it - 1
+                const bool conv = it > 0 && (it % J.check_every == 0 || it == J.maxiter) && v[0] <= q.target;
+                if (conv || it == J.maxiter) {
                     q.on = 0;
                     if (q.a == 0) {
                         J.mdone[q.m] = it;
@@ -236,11 +238,53 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
                         atomicAdd(J.nstop, 1u);
                     }
                 } else {
+                    q.ap = (it == 0 || q.gp == 0.0) ? 0.0 : v[1] / q.gp;
                     q.gp = v[1];
                 }
+            });
+            first_on = S.n > 0 && part[0].on;
+        }
+        for (int k = 0; k < S.n; k++) {
+            Part& q = part[k];
+            if (!q.on) continue;
+            const int per = q.tr / 32, first = q.a * per + ((w - q.a * per) & (kT / 32 - 1));
+            const int last = min(q.e * per, (q.rows + 31) / 32);
+            double az[kEarly], ap[kEarly], zi[kEarly], pi[kEarly];
+#pragma unroll
+            for (int j = 0; kAhead && j < kEarly; j++) {
+                const int s = first + j * (kT / 32), o = 32 * s + lane, i = q.row0 + o;
+                az[j] = ap[j] = zi[j] = pi[j] = 0.0;
+                if (s < last && o < q.rows) {
+                    row_products<SELL, HELD, 2>(J, cv, ci, q.sl, i, J.z, pc, az[j], ap[j]);
+                    zi[j] = J.z[i]; pi[j] = pc[i];
+                }
             }
-            if (done) continue;
-            const double beta = (it == 0 || rz_old == 0.0) ? 0.0 : v[1] / rz_old;
+            double beta;
+            if constexpr (MANY) {
+                beta = q.ap;
+            } else {
+                const double rz_old = q.gp;
+                double v[2];
+                totals<2>(J, q.t0, tiles_of(q), K_RR, v, tot);
+                const bool conv = it > 0 && (it % J.check_every == 0 || it == J.maxiter) && v[0] <= q.target;
+                const bool done = conv || it == J.maxiter;
+                if (k == 0 && done) first_on = false;
+                if (tid == 0) {
+                    if (done) {
+                        q.on = 0;
+                        if (q.a == 0) {
+                            J.mdone[q.m] = it;
+                            if (!conv) atomicOr(J.status, ERR_JCG_NOT_CONVERGED);
+                            __threadfence();
+                            atomicAdd(J.nstop, 1u);
+                        }
+                    } else {
+                        q.gp = v[1];
+                    }
+                }
+                if (done) continue;
+                beta = (it == 0 || rz_old == 0.0) ? 0.0 : v[1] / rz_old;
+            }
             for (int a = q.a; a < q.e; a += kTileRun) {
                 const int e = min(q.e, a + kTileRun);
                 const int s0 = a * per, s1 = min(e * per, last);
@@ -256,7 +300,7 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
                     if (o < q.rows) {
                         double s1_, s2_, z_, p_;
                         const int j = (s - first) / (kT / 32);
-                        if (HELD && j < kEarly) {
+                        if (kAhead && j < kEarly) {
                             s1_ = j ? az[1] : az[0]; s2_ = j ? ap[1] : ap[0];
                             z_ = j ? zi[1] : zi[0]; p_ = j ? pi[1] : pi[0];
                         } else {
@@ -290,13 +334,20 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
         SYNC64();
         // (uniform: nstop only changes in the set-up and in phase A, each with a barrier behind it)
         if (*((volatile unsigned*)J.nstop) >= (unsigned)nmem) break;
+        if constexpr (MANY)
+            part_totals<1>(J, S, part, K_PQ, [&](Part& q, const double (&v)[1]) { q.ap = v[0] != 0.0 ? q.gp / v[0] : 0.0; });
         for (int k = 0; k < S.n; k++) {
             const Part& q = part[k];
             if (!q.on) continue;
             const int per = q.tr / 32;
-            double v[1];
-            totals<1>(J, q.t0, tiles_of(q), K_PQ, v, tot);
-            const double alpha = v[0] != 0.0 ? q.gp / v[0] : 0.0;
+            double alpha;
+            if constexpr (MANY) {
+                alpha = q.ap;
+            } else {
+                double v[1];
+                totals<1>(J, q.t0, tiles_of(q), K_PQ, v, tot);
+                alpha = v[0] != 0.0 ? q.gp / v[0] : 0.0;
+            }
             for (int a = q.a; a < q.e; a += kTileRun) {
                 const int e = min(q.e, a + kTileRun);
                 const int s0 = a * per, s1 = min(e * per, (q.rows + 31) / 32);
@@ -332,26 +383,34 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
 
 // Kernel, grid and shared memory of a solve of `rows` rows.  A row of a triangular mesh has about seven
 // entries; the matrix is held when that many fit the blocks' shared memory (a block whose rows turn out
-// to have more reads them from global memory).
+// to have more reads them from global memory).  Batches of members below 1,024 rows on average are not held:
+// what bounds them is a block's chain of parts, which two blocks per SM halve (256 members of 400 rows 1.56 ms,
+// 1.70 held; 64 of 1,600 rows 2.74 and 2.67; 32 of 8,100 rows 6.98 and 6.76).
 struct Shape64 {
     const void* fn;
     int grid, entries;
     size_t shared;
 };
+template <bool HELD>
+static const void* kernel64(bool sell, bool many) {
+    if (!sell) return (const void*)k_jcg64<false, HELD, false>;       // a caller's matrix is one member
+    return many ? (const void*)k_jcg64<true, HELD, true> : (const void*)k_jcg64<true, HELD, false>;
+}
 static cudaError_t jcg64_shape(bool sell, long long rows, int ntiles, int nmem, int nsm, Shape64& S) {
-    S.fn = sell ? (const void*)k_jcg64<true, true> : (const void*)k_jcg64<false, true>;
+    S.grid = std::max(1, std::min(ntiles, nsm));
+    const bool many = nmem > 1 && ntiles > S.grid;
+    S.fn = kernel64<true>(sell, many);
     long long room = 0;
     cudaError_t e = grant_shared(S.fn, room);
     if (e != cudaSuccess) return e;
-    S.grid = std::max(1, std::min(ntiles, nsm));
     long long parts = (long long)(sizeof(Part) * share_parts(nmem, S.grid));
     if (parts > room) return cudaErrorInvalidConfiguration;
     S.entries = (int)((room - parts) / 12) & ~1;
-    if (rows * 7 <= (long long)S.entries * S.grid) {
+    if (!(many && rows < 1024LL * nmem) && rows * 7 <= (long long)S.entries * S.grid) {
         S.shared = (size_t)parts + 12 * (size_t)S.entries;
     } else {
-        const void* fn = sell ? (const void*)k_jcg64<true, false> : (const void*)k_jcg64<false, false>;
         const int grid = std::max(1, std::min(ntiles, 2 * nsm));
+        const void* fn = kernel64<false>(sell, nmem > 1 && ntiles > grid);
         const size_t shared = sizeof(Part) * share_parts(nmem, grid);
         int fit = 0;
         long long room2 = 0;

@@ -242,31 +242,37 @@ __device__ __forceinline__ void part_sum(const SolveView& J, const Part& q, Tile
     }
 }
 
-// Totals of kinds [k0, k0 + NV) of the n tiles from t0: the first warp adds the partials, lane by lane
-// and then over the lanes, while the other warps go on to the barrier inside.
+// Totals of kinds [k0, k0 + NV) of the n tiles from t0 in one warp: the partials are added lane by lane and
+// then over the lanes.
+template <int NV>
+__device__ __forceinline__ void lane_totals(const SolveView& J, int t0, int n, int k0, double (&s)[NV]) {
+#pragma unroll
+    for (int k = 0; k < NV; k++) s[k] = 0.0;
+    for (int t = threadIdx.x & 31; t < n; t += 128) {
+        double u[NV][4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                u[k][j] = t + 32 * j < n ? __ldcg(J.part + (size_t)(k0 + k) * J.ntiles + t0 + t + 32 * j) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int k = 0; k < NV; k++) s[k] += u[k][j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < NV; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+}
+
+// The same totals in every thread: the first warp adds them while the other warps go on to the barrier inside.
 template <int NV>
 __device__ __forceinline__ void totals(const SolveView& J, int t0, int n, int k0, double (&v)[NV], double* sh) {
     __syncthreads();
     if (threadIdx.x < 32) {
         double s[NV];
-#pragma unroll
-        for (int k = 0; k < NV; k++) s[k] = 0.0;
-        for (int t = threadIdx.x; t < n; t += 128) {
-            double u[NV][4];
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int k = 0; k < NV; k++)
-                    u[k][j] = t + 32 * j < n ? __ldcg(J.part + (size_t)(k0 + k) * J.ntiles + t0 + t + 32 * j) : 0.0;
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int k = 0; k < NV; k++) s[k] += u[k][j];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int k = 0; k < NV; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        lane_totals<NV>(J, t0, n, k0, s);
         if (threadIdx.x == 0)
 #pragma unroll
             for (int k = 0; k < NV; k++) sh[k] = s[k];

@@ -222,13 +222,31 @@ def test_timed_out_block_member_is_reported_and_the_context_recovers(native):
         ref.close()
 
 
-def test_many_small_members_do_not_wait_for_one_another(native):
-    """256 members of 400 rows take less than three times the time of one."""
+@pytest.mark.parametrize("precision,most", [("fp32_ir", 3.0), ("fp64", 2.3)])
+def test_many_small_members_do_not_wait_for_one_another(native, precision, most):
+    """256 members of 400 rows take less than `most` times the time of one (measured 1.9 in both)."""
     from gschism_b200.model import Model
     times = []
     for n in (1, 256):
-        m = Model([_basin(100 + k, 20) for k in range(n)], precision="fp32_ir")
+        m = Model([_basin(100 + k, 20) for k in range(n)], precision=precision)
         m.step(8)
         times.append(_solve_ms(m, 9))
         m.close()
-    assert times[1] <= 3.0 * times[0], times
+    assert times[1] <= most * times[0], times
+
+
+@pytest.mark.parametrize("sides", [[45, 120, 173], [20, 25, 30, 18] * 24], ids=["held", "small"])
+def test_fp64_members_of_shared_blocks_equal_their_solo_runs(native, sides):
+    """FP64 batches with more tiles than blocks, matrix held and not: bit for bit the solo results."""
+    from gschism_b200.model import Model
+    cs = [_basin(200 + k, s) for k, s in enumerate(sides)]
+    assert sum(max(1, (s * s + 255) // 256) for s in sides) > 148
+    mix = Model(cs, precision="fp64")
+    mix.step(2)
+    for k in range(0, len(cs), max(1, len(cs) // 8)):
+        solo = Model(cs[k:k + 1], precision="fp64")
+        solo.step(2)
+        assert np.array_equal(mix.get(k, "ETA2"), solo.get(0, "ETA2")), k
+        assert mix.stats(k)["jcg_iters"] == solo.stats(0)["jcg_iters"]
+        solo.close()
+    mix.close()
