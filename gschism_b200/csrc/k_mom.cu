@@ -51,10 +51,12 @@ __device__ __forceinline__ double2 slip(double2 u, int8_t bt, double nx, double 
     return t * vtan - nn * vnorm;
 }
 
-// Bound by the latency of a column's level loop (divisions that depend on the level below, and loads).  Each
-// level's inputs are loaded one level ahead of its divisions; at four blocks of 128 per SM that needs no
-// spills: 742 us on 1.08M sides of 30 levels, 892 without the loads ahead at eight blocks (with them 1,052).
-__global__ void __launch_bounds__(128, 4) k_momentum(Dev d, Phys P) {
+// Bound by the latency of a column's level loop (divisions that depend on the level below, and loads).  With
+// AHEAD each level's inputs are loaded one level ahead of its divisions; at four blocks of 128 per SM that needs
+// no spills: 742 us on 1.08M sides of 30 levels, 892 without the loads ahead at eight blocks (with them 1,052).
+// The same values in both forms.
+template <bool AHEAD>
+__global__ void __launch_bounds__(128, AHEAD ? 4 : 8) k_momentum(Dev d, Phys P) {
     const int NS = d.NS, nvrt = P.nvrt;
     const double dt = P.dt, th = P.thetai;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < NS; s += gridDim.x * blockDim.x) {
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(128, 4) k_momentum(Dev d, Phys P) {
             double bet = 0.0, cprev = 0.0;
             double2 rprev = v2(0.0, 0.0);
             // level k + 1, and what level k + 2 holds, loaded ahead of level k's divisions
-            const bool two = kb + 2 < nvrt;
+            const bool two = AHEAD && kb + 2 < nvrt;
             double2 ukp1 = two ? u2[(size_t)(kb + 2) * NS + s] : v2(0.0, 0.0);
             double2 bkp1 = two ? btu[(size_t)(kb + 2) * NS + s] : v2(0.0, 0.0);
             double zkp1 = two ? d.zc[(size_t)(kb + 2) * NS + s] : 0.0;
@@ -109,10 +111,11 @@ __global__ void __launch_bounds__(128, 4) k_momentum(Dev d, Phys P) {
                 const bool top = (k == nvrt - 1);
                 double2 ukp2 = v2(0.0, 0.0), bkp2 = v2(0.0, 0.0);
                 double zkp2 = 0.0;
-                if (k + 2 < nvrt) {
-                    const size_t ix = (size_t)(k + 2) * NS + s;
+                if (k + (AHEAD ? 2 : 1) < nvrt) {
+                    const size_t ix = (size_t)(k + (AHEAD ? 2 : 1)) * NS + s;
                     ukp2 = u2[ix]; bkp2 = btu[ix]; zkp2 = d.zc[ix];
                 }
+                if (!AHEAD) { ukp1 = ukp2; bkp1 = bkp2; zkp1 = zkp2; }
                 double alow = 0.0, cupp = 0.0, bdia = 0.0;
                 const double cff1 = 1.0;
                 const double dz_0 = zk - zkm1;
@@ -167,15 +170,17 @@ __global__ void __launch_bounds__(128, 4) k_momentum(Dev d, Phys P) {
         // sides, and the stores of u2 and of the fluxes Qh (land sides carry zero flux)
         // (the next level down is loaded ahead)
         double2 r = rtop, uabove = v2(0.0, 0.0), xn = v2(0.0, 0.0);
-        double zabove = 0.0, gn = 0.0, zn = d.zc[(size_t)(nvrt - 1) * NS + s];
+        double zabove = 0.0, gn = 0.0, zn = AHEAD ? d.zc[(size_t)(nvrt - 1) * NS + s] : 0.0;
         for (int k = nvrt - 1; k >= kb; k--) {
-            const double2 x = xn;
-            const double gam = gn, zk = zn;
-            if (k > kb) {
-                const size_t ix = (size_t)(k - 1) * NS + s;
+            double2 x = xn;
+            double gam = gn, zk = zn;
+            const int kn = AHEAD ? k - 1 : k;
+            if (kn >= kb) {
+                const size_t ix = (size_t)kn * NS + s;
                 zn = d.zc[ix];
-                if (!two_d && k - 1 > kb) { xn = u2[ix]; gn = Qh[ix + NS]; }
+                if (!two_d && kn > kb && kn < nvrt - 1) { xn = u2[ix]; gn = Qh[ix + NS]; }
             }
+            if (!AHEAD) { x = xn; gam = gn; zk = zn; }
             double2 u;
             if (k > kb) {
                 if (two_d) {
@@ -284,9 +289,16 @@ __global__ void __launch_bounds__(128, 4) k_vvel(Dev d, Phys P) {
     }
 }
 
+// Short columns in several waves of blocks: what is fetched ahead of a column's few levels does not make up for
+// half the columns in flight.  1.47M sides, with the loads ahead and without: 5 levels 263 and 230 us, 7 levels
+// 327 and 310, 9 levels 377 and 373, 12 levels 457 and 481; 270k sides: 5 levels 58 and 53, 9 levels 81 and 82;
+// 30k sides (one wave) of 4 levels 13.3 and 15.4.
+constexpr int kAheadLevels = 9, kAheadSides = 512;
+
 void launch_momentum(const Dev& d, const Phys& P, cudaStream_t st, int nsm, const LaunchTable& L) {
     const LaunchShape& s = L.k[LK_MOMENTUM];
-    k_momentum<<<grid_of(d.NS, s, nsm), s.block, 0, st>>>(d, P);
+    if (P.nvrt >= kAheadLevels || d.NS <= nsm * kAheadSides) k_momentum<true><<<grid_of(d.NS, s, nsm), s.block, 0, st>>>(d, P);
+    else k_momentum<false><<<grid_of(d.NS, s, nsm), s.block, 0, st>>>(d, P);
 }
 
 void launch_vvel(const Dev& d, const Phys& P, cudaStream_t st, int nsm, const LaunchTable& L) {
@@ -297,7 +309,7 @@ void launch_vvel(const Dev& d, const Phys& P, cudaStream_t st, int nsm, const La
 int mom_max_threads(int kernel) {
     cudaFuncAttributes a{};
     cudaError_t e = cudaErrorInvalidValue;
-    if (kernel == LK_MOMENTUM) e = cudaFuncGetAttributes(&a, k_momentum);
+    if (kernel == LK_MOMENTUM) e = cudaFuncGetAttributes(&a, k_momentum<true>);
     else if (kernel == LK_VVEL) e = cudaFuncGetAttributes(&a, k_vvel);
     return e == cudaSuccess ? a.maxThreadsPerBlock : 0;
 }
