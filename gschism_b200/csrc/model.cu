@@ -241,9 +241,11 @@ static gs_status build_member(gs_ctx* c, MemberHost& m, HostBatch& B, int mid) {
     const int NP0 = (int)B.x.size(), NE0 = (int)B.area.size(), NS0 = (int)B.len.size();
     m.np0 = NP0; m.ne0 = NE0; m.ns0 = NS0;
     m.nnz0 = (int)B.indices.size();
-    // nodes
+    // nodes; without S levels (nz = nvrt) a node no deeper than h_s would have its bed at the surface level,
+    // and the kernels need at least one layer
     for (int i = 0; i < np; i++) {
         const int o = m.pn[i];
+        if (c->cfg.nz == nvrt && !(m.depth[o] > c->cfg.h_s)) return c->fail(GS_ERR_ARG, "a node without a layer (nz = nvrt)");
         B.x.push_back(m.x[o]); B.y.push_back(m.y[o]); B.depth.push_back(m.depth[o]); B.drag.push_back(m.drag[o]);
         B.tau.push_back(m.tau[2 * o]); B.tau.push_back(m.tau[2 * o + 1]);
         B.nbnd.push_back(m.isbnd[o]);

@@ -58,7 +58,7 @@ gs_status gs_grid_build(int np, int ne, const int32_t* elnode, const int32_t* i3
 
 typedef struct {
     int nvrt, ntr;                         /* levels and tracers (shared by all members) */
-    int nz; double h_s, h_c, theta_b, theta_f;
+    int nz; double h_s, h_c, theta_b, theta_f;   /* 1 <= nz <= nvrt; nz = nvrt needs every node deeper than h_s */
     const double* ztot;                    /* [nz], ztot[nz-1] = -h_s (vgrid.in, ivcor = 2) */
     const double* sigma;                   /* [nvrt-nz+1] */
     double dt, thetai, h0, dtb_min, dtb_max, velmin_btrack, rmaxvel, dfv0, coricoef, rho0, grav, dramp;

@@ -3,6 +3,8 @@ and phase codes agree between the header, the Python front end and the oracle.""
 import os
 import re
 
+import pytest
+
 from gschism_b200 import _lib as L
 from gschism_b200.model import FIELDS
 
@@ -41,3 +43,18 @@ def test_config_struct_matches_header():
     body = txt[txt.index("typedef struct {", txt.index("-- model ----")):txt.index("} gs_config;")]
     fields = re.findall(r"\b(\w+)\s*[;,]", re.sub(r"/\*.*?\*/", "", body, flags=re.S))
     assert [f for f, _ in L.GsConfig._fields_] == fields
+
+
+def test_columns_without_a_layer_are_refused(native):
+    """All levels of a vertical grid are Z levels (nz = nvrt) and a node is no deeper than h_s: its bed would
+    be the surface level.  Refused on the host; the same members with an S layer are taken."""
+    from gschism_b200 import cases
+    from gschism_b200.model import Model
+    for nz, ok in ((3, False), (2, True)):
+        c = cases.basin(seed=3, n=12, nvrt=3, nz=nz, ntr=1, length=6000.0)
+        if ok:
+            Model([c], defer_device=True)
+            continue
+        with pytest.raises(L.GsError) as ei:
+            Model([c], defer_device=True)
+        assert ei.value.status == L.GS_ERR_ARG
