@@ -596,9 +596,12 @@ __global__ void __launch_bounds__(kGatherThreads) k_nodal_tracer(Dev d, Phys P) 
     }
 }
 
-// All tracers of a column in one thread when there are columns enough to fill the GPU's threads (heights
-// and fluxes are then read once), one tracer per thread below that: 40k nodes, 40 levels, 5 tracers 198 us.
-constexpr int kColumnsPerSM = 2048;
+// All tracers of a column in one thread when there are columns enough to keep the SMs busy (heights and fluxes
+// are then read once), one tracer per thread below that.  The whole transport step, one tracer and all per
+// thread, us: 10k elements of 40 levels, 5 tracers, TVD 200 and 253; 20k elements of 23 levels, 3 tracers, FCT
+// 191 and 236; 51k elements of 30 levels, 2 tracers, upwind 135 and 141, of 40 levels, 5 tracers, TVD 647 and
+// 660; 79k elements, the same two, 205 and 195, 970 and 946; 179k elements 389 and 369, 2,190 and 2,077.
+constexpr int kColumnsPerSM = 448;
 
 template <int NTR, bool TVD, bool FCT>
 static void launch_vertical(const Dev& d, const Phys& P, double dt, cudaStream_t st, int nsm) {

@@ -1,6 +1,6 @@
 """The transport step's forms (gpu): a member's tracers are the same bits whatever form its batch takes.
 
-The vertical sweep takes one tracer per thread below about 300,000 elements and all tracers of a column
+The vertical sweep takes one tracer per thread below about 66,000 elements and all tracers of a column
 above; the horizontal update made with the whole remaining time is made again for members whose
 admissible sub-step is shorter.  Both depend on the batch, the arithmetic does not."""
 import numpy as np
