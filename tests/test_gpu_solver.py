@@ -119,3 +119,61 @@ def test_solvers_of_two_threads_do_not_disturb_each_other(native):
         assert isinstance(results[k], list), results[k]
         assert s.checkSolution() <= 1e-9
         s.close()
+
+
+def _banded(n, offsets):
+    """CSR of a symmetric diagonally dominant matrix: -1 at the offsets (both sides), rows summing to 0.5, so
+    its eigenvalues lie in [0.5, 4 len(offsets) + 0.5]."""
+    off = np.array(sorted([-o for o in offsets] + [0] + list(offsets)))
+    c = np.arange(n)[:, None] + off
+    keep = (c >= 0) & (c < n)
+    deg = keep.sum(1)
+    ptr = np.zeros(n + 1, dtype=np.int32)
+    ptr[1:] = np.cumsum(deg)
+    v = np.where(off == 0, (deg - 1)[:, None] + 0.5, -1.0)
+    return ptr, c[keep].astype(np.int32), v[keep]
+
+
+_NEIGHBOURS = (1, 389)                                      # a lattice of 389 columns
+_DENSE = tuple(range(1, 16))                                # 31 entries a row
+
+
+@pytest.mark.parametrize("n,offsets,precision", [
+    (151321, _NEIGHBOURS, "fp64"), (151321, _NEIGHBOURS, "fp32_ir"),      # several tiles and rows a thread
+    (40001, _NEIGHBOURS, "fp64"), (40001, _NEIGHBOURS, "fp32_ir"),        # one slice a warp, ragged end
+    (409601, _NEIGHBOURS, "fp64"), (640001, _NEIGHBOURS, "fp32_ir"),      # beyond the chip's shared memory
+    (151321, _DENSE, "fp64"), (151321, _DENSE, "fp32_ir"),                # a block's rows do not fit its cache
+    (1, (1,), "fp64"), (1, (1,), "fp32_ir"), (33, (1,), "fp64"), (33, (1,), "fp32_ir")])
+def test_csr_forms_against_known_solution(native, n, offsets, precision):
+    """Every form of the stand-alone solves against the solution the right-hand side was made from.  The solve
+    stops at |r| <= 1e-12 |b|, so |x - x*| <= 1e-12 |b| / 0.5 <= 1e-12 (4 len(offsets) + 0.5) / 0.5 |x*|; the
+    right-hand side is exact to rounding (1e-15 of the same factor)."""
+    from gschism_b200.solver import PCGSolverMultiGPU
+    ptr, idx, val = _banded(n, offsets)
+    truth = np.random.default_rng(n).standard_normal(n)
+    rows = np.repeat(np.arange(n), np.diff(ptr))
+    b = np.bincount(rows, weights=val * truth[idx], minlength=n)
+    s = PCGSolverMultiGPU(None, [n], [val.size], precision=precision)
+    _fill(s, (ptr, idx, val), b)
+    bound = 1.1e-12 * (4 * len(offsets) + 0.5) / 0.5
+    for check in (10, 7):                                   # the second solve starts from its own history
+        its = s.solve(rtol=1e-12, maxiter=600, checkEvery=check)
+        assert 0 < its < 600 or check == 7
+        x = s.x_m[0].cpu().numpy()
+        assert np.linalg.norm(x - truth) <= bound * np.linalg.norm(truth)
+        assert s.checkSolution() <= 1.01e-12
+    s.close()
+
+
+@pytest.mark.parametrize("n", [33, 40001])
+def test_csr_zero_rhs_mixed_precision(native, n):
+    """A zero right-hand side is answered with x = 0 and no iteration, also after a solve."""
+    from gschism_b200.solver import PCGSolverMultiGPU
+    A = _banded(n, _NEIGHBOURS)
+    s = PCGSolverMultiGPU(None, [n], [A[2].size], precision="fp32_ir")
+    for b in (np.zeros(n), np.ones(n), np.zeros(n)):
+        _fill(s, A, b)
+        its = s.solve(rtol=1e-12, maxiter=600)
+        assert (its == 0) == (not b.any())
+        assert b.any() or np.all(s.x_m[0].cpu().numpy() == 0.0)
+    s.close()
