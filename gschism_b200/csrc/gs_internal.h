@@ -117,7 +117,7 @@ struct Dev {
     int32_t *row_at32;
     // JCG vectors
     double *b, *xs, *r, *zz, *p0, *p1, *q, *invD, *xh0, *xh1, *xh2;
-    float *ir32, *diag32;          // ir32: kIrVectors FP32 vectors of the refinement solve
+    float *ir32, *diag32;          // ir32: kMgVectors FP32 vectors of the refinement solve
     // sides
     int32_t *sn, *se;              // [2][NS]
     double *len, *snx, *sny, *scx, *scy, *cori;

@@ -1,8 +1,8 @@
-// Work list of the elevation solves and their dispatch (jcg64.cu: FP64; jcg_mg.cu: mixed precision of a
-// context; jcg_ir.cu: mixed precision of a caller's CSR matrix).
+// Work list of the elevation solves and their dispatch (jcg64.cu: FP64; jcg_mg.cu and, for small members,
+// jcg_small.cu: mixed precision of a context; jcg_ir.cu: mixed precision of a caller's CSR matrix).
 //
-// A member's rows are cut into tiles whose size depends only on that member's row count; every reduction
-// adds one partial per tile in tile order.  Sums are therefore deterministic and independent of the
+// A member's rows are cut into tiles whose size depends only on that member's row count; every grid-wide
+// reduction adds one partial per tile in tile order.  Sums are therefore deterministic and independent of the
 // batch composition: a member gives bit-identical results alone and inside any batch.  Scalars stay on
 // the device; convergence is tested on the device, so a solve never returns to the host.
 #include <algorithm>
@@ -49,8 +49,8 @@ cudaError_t jcg_work_alloc(JcgWork*& w, const std::vector<int>& row0, const std:
     A((void**)&w->mem_ab, 64 * nm);
     A((void**)&w->mctl, 4 * (6 * nm + 4));
     if (e != cudaSuccess) return e;
-    w->mdone = w->mctl; w->mouter = w->mctl + nm; w->minner = w->mctl + 2 * nm; w->mret = w->mctl + 3 * nm;
-    w->mgen = w->mctl + 4 * nm; w->mcnt = (unsigned*)(w->mctl + 5 * nm);
+    w->mdone = w->mctl; w->mouter = w->mctl + nm; w->minner = w->mctl + 2 * nm; w->mbad[0] = w->mctl + 3 * nm;
+    w->mgen = w->mctl + 4 * nm; w->mbad[1] = w->mctl + 5 * nm;
     w->ndone = (unsigned*)(w->mctl + 6 * nm);
     w->status = w->mctl + 6 * nm + 1;
     w->bar = (unsigned*)(w->mctl + 6 * nm + 2);

@@ -17,7 +17,6 @@ struct gs_jcg {
     double *A = nullptr, *b = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *q = nullptr, *p0 = nullptr,
            *p1 = nullptr, *invD = nullptr, *x0 = nullptr, *x1 = nullptr, *x2 = nullptr, *scratch = nullptr;
     float *A32 = nullptr, *ir32 = nullptr, *diag32 = nullptr;
-    unsigned *bar = nullptr;
     int32_t* err = nullptr;
     JcgWork* w = nullptr;
     std::vector<void*> allocs;
@@ -97,7 +96,7 @@ gs_status gs_jcg_create(int n, int nnz, int precision, int device, gs_jcg** out)
     J(indptr, n + 1); J(indices, nnz); J(A, nnz); J(A32, nnz);
     J(b, n); J(x, n); J(r, n); J(z, n); J(q, n); J(p0, n); J(p1, n); J(invD, n); J(x0, n); J(x1, n); J(x2, n);
     J(scratch, 2); J(ir32, (size_t)kIrVectors * n); J(diag32, n);
-    J(bar, 2); J(err, 1);
+    J(err, 1);
 #undef J
     if (e == cudaSuccess) e = jcg_work_alloc(s->w, std::vector<int>{0}, std::vector<int>{n}, false, s->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
@@ -135,7 +134,7 @@ gs_status gs_jcg_solve_csr(gs_jcg* s, double rtol, int maxiter, int check_every,
     a.x = s->x; a.r = s->r; a.z = s->z; a.q = s->q; a.p0 = s->p0; a.p1 = s->p1;
     a.ir32 = s->ir32;
     a.diag32 = s->diag32;
-    a.bar = s->bar; a.err = s->err;
+    a.err = s->err;
     a.rtol = rtol; a.maxiter = maxiter; a.check_every = check_every < 1 ? 1 : check_every;
     a.inner_rtol = 0.1; a.inner_maxiter = 400;
     a.wait_polls = kWaitPolls; a.stall_member = -1;
@@ -150,8 +149,7 @@ gs_status gs_jcg_solve_csr(gs_jcg* s, double rtol, int maxiter, int check_every,
     cudaStreamSynchronize(s->st);
     if (iters) *iters = it[0];
     if (flags & ERR_BARRIER_TIMEOUT) {
-        // the barrier word is left mid-round; both words are cleared so the next solve starts clean
-        cudaMemsetAsync(s->bar, 0, sizeof(unsigned), s->st);
+        // cleared, so the next solve starts clean (it clears its control words, the barrier's among them)
         cudaMemsetAsync(s->err, 0, sizeof(int32_t), s->st);
         cudaStreamSynchronize(s->st);
         s->msg = "device barrier timed out";

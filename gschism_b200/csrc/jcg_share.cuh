@@ -79,7 +79,7 @@ struct Part {
 
 // The tiles of a sweep are dealt to the blocks over the members still active, so that the blocks stay
 // evenly loaded as members converge.  A member counts as its rows plus one eighth of a block's share:
-// that bounds the members of a block (11 and one per gridDim members), whose parts are found once per
+// that bounds the members of a block (share_parts), whose parts are found once per
 // sweep and kept in shared memory; looking them up in every phase would cost a chain of dependent
 // loads each time.
 struct Share {

@@ -15,13 +15,13 @@ struct JcgWork {
     // per member: first tile, first row, rows, rows per tile
     int32_t *mem_t0 = nullptr, *mem_row0 = nullptr, *mem_rows = nullptr, *mem_tr = nullptr;
     double *tile_part = nullptr, *mem_atol2 = nullptr, *mem_ab = nullptr;
-    // per-member control words in one array: mdone, mouter, minner, mret, mgen, mcnt ([nmem] each),
+    // per-member control words in one array: mdone, mouter, minner, mbad[0], mgen, mbad[1] ([nmem] each),
     // ndone, status (ERR_JCG_NOT_CONVERGED of the last solve), bar (grid barrier), nlev (members
     // iterating with the coarse correction)
     int32_t* mctl = nullptr;
     int32_t* status = nullptr;
-    int32_t *mdone = nullptr, *mouter = nullptr, *minner = nullptr, *mret = nullptr, *mgen = nullptr;
-    unsigned* mcnt = nullptr;
+    int32_t *mdone = nullptr, *mouter = nullptr, *minner = nullptr, *mgen = nullptr;
+    int32_t* mbad[2] = {nullptr, nullptr};
     unsigned *ndone = nullptr, *bar = nullptr, *nlev = nullptr;
 };
 

@@ -412,7 +412,10 @@ __device__ __forceinline__ void for_runs(const Dev& d, int nvrt, int groups, F f
 }
 
 // Upwind shares the faces' fluxes between the tracers; with TVD the limiters dominate, and a work item
-// takes one tracer (fewer registers, more threads).
+// takes one tracer (more threads).  At 64 registers both spill (upwind 56 to 200 bytes of stores, TVD 396 to
+// 460), and four blocks per SM are still the best split: the transport step of 40k nodes, 40 levels, 5
+// tracers, TVD takes 970 us at four, 1,028 at three and 1,196 at two; of 250k nodes, 30 levels, upwind 637, 695
+// and 826.
 template <int NTR, bool TVD>
 __global__ void __launch_bounds__(256, 4) k_transport(Dev d, Phys P, TrArgs T) {
     constexpr int NT = TVD ? 1 : NTR, groups = NTR / NT;
@@ -539,7 +542,7 @@ cudaError_t launch_tracer_mass(const Dev& d, const Phys& P, int e0, int e1, doub
 
 // levels of a node that one thread sums
 template <int NTR>
-constexpr int nodal_run() { return NTR <= 2 ? 3 : (NTR <= 4 ? 3 : 2); }
+constexpr int nodal_run() { return NTR <= 4 ? 3 : 2; }
 
 // nodalTracerUpdate, meshdata.cu:6739-6774 (node-centred gather, no atomics).  A thread owns a run of
 // levels of one node, run in blockIdx.y: an element's index, wetness, area and bed are looked up once

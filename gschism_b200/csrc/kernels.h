@@ -19,10 +19,9 @@ struct JcgArgs {
     const float* A32;                    // D^-1 A in FP32
     const double *b, *invD;
     double *x, *r, *z, *q, *p0, *p1;
-    float* ir32;                         // kIrVectors * n floats
+    float* ir32;                         // kMgVectors (a context) or kIrVectors (a caller's matrix) * n floats
     const float* diag32;                 // matrix diagonal in FP32
     const MgDev* mg;                     // hierarchy of a context's refinement solve
-    unsigned* bar;
     int32_t* err;
     double rtol;
     int maxiter, check_every;

@@ -685,7 +685,7 @@ static gs_status run_phase(gs_ctx* c, int phase, int arg) {
         a.indptr = nullptr; a.sell = d.sell; a.indices = d.indices; a.A = d.A; a.A32 = nullptr; a.mg = &c->mg; a.b = d.b; a.invD = d.invD;
         a.x = d.xs; a.r = d.r; a.z = d.zz; a.q = d.q; a.p0 = d.p0; a.p1 = d.p1;
         a.ir32 = d.ir32; a.diag32 = d.diag32;
-        a.bar = d.bar; a.err = d.err;
+        a.err = d.err;
         a.rtol = c->cfg.rtol; a.maxiter = c->cfg.maxiter; a.check_every = c->cfg.check_every;
         a.inner_rtol = c->cfg.ir_inner_rtol; a.inner_maxiter = c->cfg.ir_inner_maxiter;
         a.wait_polls = c->d.wait_polls; a.stall_member = c->stall_member;

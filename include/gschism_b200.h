@@ -213,8 +213,7 @@ gs_status gs_get_step(gs_ctx* ctx, int* step);
 
 /* Device memory a context holding members of these sizes allocates (bytes, an upper bound used
    for admission by HBM footprint).  np/ne/ns/nnz are the sums over the members.  A TVD context
-   (itr_met = 3) allocates ne * nvrt * ntr * 8 bytes more, one with the vertical FCT (itr_met = 4)
-   ne * nvrt * (ntr + 1) * 8 bytes more. */
+   (itr_met = 3 or 4) allocates ne * nvrt * ntr * 8 bytes more. */
 size_t gs_footprint_bytes(int nvrt, int ntr, int nmem, int64_t np, int64_t ne, int64_t ns, int64_t nnz);
 
 typedef struct {
@@ -249,8 +248,8 @@ gs_status gs_get_launch(gs_ctx* ctx, int kernel, int* a, int* b);
    budget; this is the FP64 budget the mass-conservation checks read. */
 gs_status gs_tracer_mass(gs_ctx* ctx, int member, double* out);
 
-/* Bound of every device wait of the context's persistent kernels (the grid barrier of the
- * transport and the solver's member-level waits), in polls: after 4,096 plain polls each poll
+/* Bound of every device wait of the context's persistent kernels (the grid barriers of the
+ * transport and of the solves), in polls: after 4,096 plain polls each poll
  * sleeps about 128 ns, so the default (0 selects it: 2^24 polls) is about 2 s.  A wait that runs
  * out sets a flag; every block then leaves its kernel, later launches of the step return at
  * once, and the next gs_sync / gs_get_stats / gs_state_get returns GS_ERR_TIMEOUT and clears the

@@ -6,10 +6,8 @@ run (their device memory is handed out by their own pool, or allocation latency 
 in their loop); its work space is a fixed array inside the library that every call reuses, so the
 second call checks that nothing left over from the first one leaks into the result.
 
-The allocation-free solve cuts rows into 256-row tiles and the allocating one into tiles of at
-least 1,024 rows, so their dot products add partial sums in different orders: solutions agree to
-the solver tolerance (1e-10 relative at rtol 1e-12), and iteration counts by up to one test
-interval (check_every).  Systems: the 10 km channel (2,016 rows) and a 250 x 250 basin (62,500
+Both cut rows into tiles of 256 rows at these sizes.  Solutions are held to the solver tolerance
+(1e-10 relative at rtol 1e-12), iteration counts to one test interval (check_every).  Systems: the 10 km channel (2,016 rows) and a 250 x 250 basin (62,500
 rows, close to the 65,536-row limit), from a zero and from a nonzero initial guess.
 """
 import ctypes
