@@ -63,7 +63,7 @@ struct MgView : SolveView {
     int32_t *mdone, *mouter, *minner;        // results: iterations (-1: not converged), sweeps, iterations
     int32_t* mbad[2];                        // by sweep parity: sweeps that did not halve the residual
     unsigned* nstop;                         // members not iterating in this sweep
-    unsigned* nlev;                          // members iterating with the coarse correction
+    unsigned* nlev;                          // members that iterate with the coarse correction in this sweep
     int32_t* status;
     int stall_member;
     double rtol, inner_rtol;
@@ -430,10 +430,13 @@ __device__ __forceinline__ RowVec row_vec(const MgView& J, const Part& q, int i)
     return {q.lev ? J.z[i] : J.u[i], J.w[i], J.p[i], J.s[i], J.d[i], J.u[i], __ldcg(J.diag + i)};
 }
 
-// (no thread leaves the kernel with copies of its own in flight)
-#define MG_SYNC() do { if (!bar.sync(J, stall)) { ring_drain(); return; } } while (0)
+// A failed wait ends the kernel; no thread leaves with copies of its own in flight.  (Predicated in PTX: as a
+// branch of its own behind each of the fourteen barriers it costs registers, and 3% of the solve.)
+__device__ __forceinline__ void leave_unless(bool ok) {
+    asm volatile("{ .reg .pred p; setp.eq.s32 p, %0, 0; @p cp.async.wait_all; @p exit; }" ::"r"((int)ok) : "memory");
+}
+#define MG_SYNC() leave_unless(bar.sync(J, stall))
 
-// (64 registers for two blocks per SM; 120 bytes of spill stores and 208 of loads)
 __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
     __shared__ double sh[3][kT / 32];
     __shared__ TileSums ts;
@@ -481,7 +484,7 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
     for (int sweep = 0; sweep < 64; sweep++) {
         const int par = sweep & 1;
         mg_share(J, sweep, S, part, member_on);
-        if (S.none) break;         // no member left (every block agrees)
+        if (S.none) { ring_drain(); break; }
         // O1: r = b - A x; u = D^-1 r in FP32 replaces the recursive residual, d = 0
         for (int k = 0; k < S.n; k++) {
             const Part& q = part[k];
@@ -561,21 +564,21 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
             }
         }
         __syncthreads();
-        // The cycle runs while a member iterates with it: members that iterate longer without it do not
-        // pay for its eight barriers (a plain iteration takes 7 to 10 us, one with the cycle 30 to 40).
-        // nstop and nlev are read behind a barrier after O2 or F2, which alone change them, so every block
-        // reads the same values.
-        bool cycle = with_levels != 0;
-        for (int it = 0; it <= J.inner_maxiter; it++) {
-            if (cycle) {
-                level_down<0>(J, member_on, R);
-                level_open<1>(J, member_on, R);
-            }
-            if (cycle || it == 0) MG_SYNC();
-            if (it == 0) {
-                if (*((volatile unsigned*)J.nstop) >= (unsigned)nmem) break;
-                cycle = *((volatile unsigned*)J.nlev) > 0u;
-            }
+        // The cycle runs in a sweep in which a member iterates with it; one in which none does goes on without its
+        // eight barriers (a plain iteration takes 7 to 10 us, one with the cycle 30 to 40).  The cycle's first phase
+        // stands at the end of the iteration before, and the loop is skipped by its counter: in this form the
+        // kernel's 64 registers suffice (-Xptxas -v: no spills; 160k rows 2.70 ms a solve), with the phase at the
+        // start or a break instead it spills 120 bytes (2.79 to 2.90).  nstop and nlev are read behind a barrier
+        // after O2 or F2, which alone change them, so every block reads the same values.
+        if (with_levels) {
+            level_down<0>(J, member_on, R);
+            level_open<1>(J, member_on, R);
+        }
+        MG_SYNC();
+        const bool cycle = *((volatile unsigned*)J.nlev) > 0u;
+        int it = 0;
+        if (*((volatile unsigned*)J.nstop) >= (unsigned)nmem) it = J.inner_maxiter + 1;      // every member has converged
+        for (; it <= J.inner_maxiter; it++) {
             if (cycle) {
                 level_down<1>(J, member_on, R);
                 level_open<2>(J, member_on, R);
@@ -643,7 +646,6 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
                             J.minner[m] += it;
                             __threadfence();
                             atomicAdd(J.nstop, 1u);
-                            if (q.lev) atomicSub(J.nlev, 1u);
                         }
                     } else {
                         q.ap = alpha; q.gp = v[0];
@@ -670,7 +672,11 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
             if (cycle) level_open<0>(J, member_on, R);
             MG_SYNC();
             if (*((volatile unsigned*)J.nstop) >= (unsigned)nmem) break;
-            cycle = *((volatile unsigned*)J.nlev) > 0u;
+            if (cycle) {
+                level_down<0>(J, member_on, R);
+                level_open<1>(J, member_on, R);
+                MG_SYNC();
+            }
         }
         // x += d for the members that iterated in this sweep
         for (int k = 0; k < S.n; k++) {
@@ -680,7 +686,6 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
         }
         MG_SYNC();
     }
-    ring_drain();
     for (int m = blockIdx.x * kT + tid; m < nmem; m += gridDim.x * kT)
         if (*((volatile int32_t*)&J.mdone[m]) < 0) {
             J.mdone[m] = J.minner[m];

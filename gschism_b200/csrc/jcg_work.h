@@ -17,7 +17,7 @@ struct JcgWork {
     double *tile_part = nullptr, *mem_atol2 = nullptr, *mem_ab = nullptr;
     // per-member control words in one array: mdone, mouter, minner, mbad[0], mgen, mbad[1] ([nmem] each),
     // ndone, status (ERR_JCG_NOT_CONVERGED of the last solve), bar (grid barrier), nlev (members
-    // iterating with the coarse correction)
+    // that iterate with the coarse correction in a sweep)
     int32_t* mctl = nullptr;
     int32_t* status = nullptr;
     int32_t *mdone = nullptr, *mouter = nullptr, *minner = nullptr, *mgen = nullptr;

@@ -115,12 +115,13 @@ def test_values_written_in_the_launch_are_read_coherently():
 
 
 def test_no_exit_with_copies_in_flight():
-    """Every way out of the solve's kernel waits for the thread's own asynchronous copies first: slices are
-    requested before the barrier that may end the kernel."""
+    """Every way out of the solve's kernel behind the first barrier waits for the thread's own asynchronous
+    copies: slices are requested before the barrier that may end the kernel."""
     text = open(os.path.join(CSRC, "jcg_mg.cu")).read()
     body = text[text.index("__global__"):text.index("static size_t mg_shared")]
-    sync = re.search(r"#define MG_SYNC\(\) (.*)", text).group(1)
-    assert re.search(r"ring_drain\(\);\s*return", sync)
-    assert "return;" not in body                       # the macro is the only early exit
-    loop = body[body.index("for (int sweep"):]
-    assert "ring_drain();" in loop[loop.rindex("MG_SYNC"):]
+    assert "leave_unless(bar.sync(J, stall))" in re.search(r"#define MG_SYNC\(\) (.*)", text).group(1)
+    leave = text[text.index("void leave_unless"):]
+    assert re.search(r"@p cp\.async\.wait_all; @p exit;", leave[:leave.index("\n}")])
+    loop = body[body.index("MG_SYNC"):]
+    assert "return;" not in loop                        # a failed wait is the only early exit
+    assert re.search(r"if \(S\.none\) \{ ring_drain\(\); break; \}", loop)
