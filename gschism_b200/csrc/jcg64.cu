@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg64(View64 J) {
     int32_t* const ci = reinterpret_cast<int32_t*>(cv + J.cache_entries);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nmem = J.nmem;
     const bool stall = J.stall_member >= 0 && blockIdx.x == 0;
+    if (__syncthreads_or(timed_out(J.err))) return;
     GridBarrier bar;
     make_share(J, 0, S, part, [](Part&) {});
     // the matrix entries of the block's parts, as many parts as fit (Part::sl: their shift)

@@ -450,6 +450,7 @@ __global__ void __launch_bounds__(kT, 2) k_jcg_mg(MgView J, int with_levels) {
     uint8_t* const member_on = reinterpret_cast<uint8_t*>(part + J.max_parts);
     const int tid = threadIdx.x, nmem = J.nmem;
     const bool stall = J.stall_member >= 0 && blockIdx.x == 0;
+    if (__syncthreads_or(timed_out(J.err))) return;
     GridBarrier bar;
     // |b|^2 partials; coarse matrices of this step's A
     mg_share(J, 0, S, part, member_on);

@@ -45,6 +45,12 @@ struct GridBarrier {
     }
 };
 
+// A launch that starts after a wait ran out in an earlier one (the host has not reported and cleared it yet)
+// leaves at once: its inputs are those of an unfinished step.
+__device__ __forceinline__ bool timed_out(const int32_t* err) {
+    return (*((const volatile int32_t*)err) & ERR_BARRIER_TIMEOUT) != 0;
+}
+
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[kT / 32]) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

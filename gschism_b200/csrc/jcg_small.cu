@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(kT) k_jcg_small(SmallView J) {
     __shared__ double sh[3][kT / 32];
     __shared__ float us[kMgMinRows];
     if (tid == 0) J.mfin[m] = -1;            // not among the members that iterate together
+    if (__syncthreads_or(timed_out(J.err))) return;
     if (m == J.stall_member) {
         // recovery tests: a wait that runs out
         if (tid == 0) {

@@ -73,3 +73,29 @@ def test_not_converged_is_reported_per_solve(native):
         assert m.stats(0)["error_flags"] == 0
     finally:
         m.close()
+
+
+@pytest.mark.parametrize("precision,size", [("fp64", (63, 32)), ("fp32_ir", (63, 32)), ("fp32_ir", (31, 16))])
+def test_solve_after_a_timed_out_one_leaves_at_once(native, precision, size):
+    """Until the host has reported a timeout, later launches of the step return without working on the state
+    of the unfinished one: the second solve, no longer stalled, makes no iteration."""
+    import ctypes
+    from gschism_b200.model import Model
+    m = Model([cases.channel(seed=3, nx=size[0], ny=size[1])], precision=precision)
+    try:
+        m.step(2)
+        assert m.stats(0)["jcg_iters"] > 0
+        m.set_wait_limit(1 << 14)
+        for ph in ("BEGIN", "BTRACK", "PREPARE", "ASSEMBLE"):
+            m.phase(ph, 3)
+        m.test_stall_solve(0)
+        m.phase("SOLVE", 3)
+        m.test_stall_solve(-1)
+        m.phase("SOLVE", 3)
+        out = L.GsStats()
+        assert m.lib.gs_get_stats(m.h, 0, ctypes.byref(out)) == L.GS_ERR_TIMEOUT
+        assert out.jcg_iters == -1
+        m.phase("SOLVE", 3)                 # reported and cleared: solves again
+        assert m.stats(0)["jcg_iters"] > 0 and m.stats(0)["error_flags"] == 0
+    finally:
+        m.close()
