@@ -140,6 +140,12 @@ class Clocks:
         return out
 
 
+# DRAM bytes (dram__bytes.sum) per iteration of k_jcg_mg on the 1M-node basin, from one ncu capture of its solve
+# (launch bytes / iterations of that launch, refinement sweeps included; profiles/); scaled below by
+# the timed launches' iterations.
+JCG_DRAM_BYTES_PER_ITER = 92.7e6
+
+
 def _jcg_bytes_per_iter(N, nnz, mode):
     """Algorithmic bytes of one iteration.  FP64 (Jacobi-PCG): matrix values + column indices + row
     pointers, and seven vector passes (read p, invD, x, r; write x, r, p).  Mixed precision (FP32
@@ -277,12 +283,12 @@ def run_ours(a):
         "e2e": r["e2e"],
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
-                     "traffic": None, "kernel": "k_jcg_mg",
+                     "traffic": JCG_DRAM_BYTES_PER_ITER * it_in, "kernel": "k_jcg_mg",
                      "peak_kind": peak_kind, "iters_per_launch": it_in, "bytes_per_launch": bytes_launch},
         "clocks": r["clocks"],
         # per step, issued phase by phase: clock, btrack, elevation BC, side preparation, ghat, assembly,
-        # solve, elevation update, momentum, vertical velocity, transport, nodal tracers, 6 level kernels,
-        # 2 density kernels (two tracers), nodal velocities (the launch list in profiles/)
+        # solve, elevation update, momentum, vertical velocity, transport (horizontal, vertical), nodal tracers,
+        # 6 level kernels, 2 density kernels (two tracers), nodal velocities (the launch list in profiles/)
         "gpu_launches": a.steps * 22,
         "jcg": {"inner_iters": r["jcg_iters_last"], "outer": r["jcg_outer_last"], "ms_avg": jms_avg},
     }

@@ -182,7 +182,8 @@ __device__ void vertical_fct(const Dev& d, const Phys& P, int e, double dt, cons
 // The eliminated super-diagonal goes to the group's own scratch slice: prev's where upwind leaves it
 // free (its values are read before they are overwritten), the inflow sums' with TVD.  The next level's
 // inputs are loaded ahead of a level's two dependent divisions.  720k columns of 30 levels, 2 tracers:
-// 386 us for 2.0 GB, 0.8 of the measured copy rate; with the column in shared memory, which moves half of
+// 386 us for 2.0 GB of loads and stores, some of which the L2 serves (318k columns: DRAM at 0.43 of the measured
+// copy rate, a third of the warps, waiting for loads); with the column in shared memory, which moves half of
 // that, 531 us (too few threads fit).
 template <int NT, bool TVD, bool FCT>
 __global__ void __launch_bounds__(128) k_vertical(Dev d, Phys P, const int32_t* nsub, double dt) {
