@@ -31,7 +31,7 @@ cudaError_t jcg_work_alloc(JcgWork*& w, const std::vector<int>& row0, const std:
     std::vector<int32_t> mt0(nmem), mtr(nmem);
     int T = 0;
     for (int m = 0; m < nmem; m++) {
-        if (rows[m] < kMgMinRows) w->nsmall++;
+        if (rows[m] < kMgMinRows) { w->nsmall++; w->small_rows = std::max(w->small_rows, rows[m]); }
         mtr[m] = tile_rows_for(rows[m], tiling);
         mt0[m] = T;
         T += (rows[m] + mtr[m] - 1) / mtr[m];

@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(kT, HELD ? 1 : 2) k_jcg_ir(View32 J) {
     int32_t* const ci = reinterpret_cast<int32_t*>(cv + J.cache_entries);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const bool stall = J.stall_member >= 0 && blockIdx.x == 0;
-    if (__syncthreads_or(timed_out(J.err))) return;
     GridBarrier bar;
     make_share(J, 0, S, part, [](Part&) {});
     const bool mine = S.n > 0;

@@ -3,10 +3,10 @@
 // PCGSolverMultiGPU.solve, src/solver/pcg_solver.py:1075-1124, whose stopping test r.r <= (rtol |b|)^2 it
 // keeps in FP64.)
 //
-// Such a member is bound by the latency of its 130 to 210 iterations, not by work: in a block of its own an
-// iteration needs no grid barrier, its vectors stay in registers and the gathered one in shared memory, and
-// members do not wait for one another.  400 rows 0.20 ms a solve, 0.93 as plain Jacobi between the grid
-// barriers of jcg_mg.cu; 256 members of 400 rows 0.37 and 4.7 ms.
+// Such a member is bound by the latency of its 100 to 400 iterations, not by work: in a block of its own an
+// iteration needs no grid barrier (1.5 us at 400 rows, 4.6 at 4,000), its vectors stay in registers and the
+// gathered one in shared memory, and members do not wait for one another.  400 rows 0.20 ms a solve, 0.93 as
+// plain Jacobi between the grid barriers of jcg_mg.cu; 256 members of 400 rows 0.37 and 4.7 ms.
 //
 // The recurrence is that of jcg_mg.cu (Chronopoulos and Gear, 1989) with z = u = D^-1 r.  Sums are taken in
 // a fixed order that depends on the member's row count alone, so a member gets the same bits alone and in
@@ -18,8 +18,6 @@
 namespace gs {
 
 namespace {
-
-constexpr int kOwn = (kMgMinRows + kT - 1) / kT;     // rows of a thread
 
 struct SmallView {
     const int32_t *row0, *rows;
@@ -37,11 +35,14 @@ struct SmallView {
     int inner_maxiter;
 };
 
+// kOwn: rows of a thread (tid, tid + 512, ...), enough for the context's largest small member; a thread's rows
+// beyond a member's end add zeros, so a member gets the same bits in every form.
+template <int kOwn>
 __global__ void __launch_bounds__(kT) k_jcg_small(SmallView J) {
     const int m = blockIdx.x, n = J.rows[m], r0 = J.row0[m], tid = threadIdx.x;
     if (n >= kMgMinRows) return;
     __shared__ double sh[3][kT / 32];
-    __shared__ float us[kMgMinRows];
+    __shared__ float us[kOwn * kT];
     if (tid == 0) J.mfin[m] = -1;            // not among the members that iterate together
     if (__syncthreads_or(timed_out(J.err))) return;
     if (m == J.stall_member) {
@@ -185,7 +186,11 @@ cudaError_t jcg_small_launch(const JcgArgs& a, JcgWork* w, cudaStream_t st) {
     J.polls = a.wait_polls > 0 ? a.wait_polls : kWaitPolls;
     J.stall_member = a.stall_member;
     J.rtol = a.rtol; J.inner_rtol = a.inner_rtol; J.inner_maxiter = a.inner_maxiter;
-    k_jcg_small<<<w->nmem, kT, 0, st>>>(J);
+    // the fewest rows a thread that hold the largest small member (400 rows: 0.19 ms with two, 0.24 with eight)
+    static_assert(kMgMinRows <= 8 * kT, "rows of a thread");
+    if (w->small_rows <= 2 * kT) k_jcg_small<2><<<w->nmem, kT, 0, st>>>(J);
+    else if (w->small_rows <= 4 * kT) k_jcg_small<4><<<w->nmem, kT, 0, st>>>(J);
+    else k_jcg_small<8><<<w->nmem, kT, 0, st>>>(J);
     return cudaGetLastError();
 }
 

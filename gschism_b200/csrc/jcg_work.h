@@ -10,7 +10,7 @@ struct JcgArgs;
 
 struct JcgWork {
     int nmem = 0, ntiles = 0;
-    int nsmall = 0;                  // members below kMgMinRows rows
+    int nsmall = 0, small_rows = 0;  // members below kMgMinRows rows, rows of the largest of them
     bool sell = false;               // rows in the SELL-32 layout of a context, else a caller's CSR
     // per member: first tile, first row, rows, rows per tile
     int32_t *mem_t0 = nullptr, *mem_row0 = nullptr, *mem_rows = nullptr, *mem_tr = nullptr;

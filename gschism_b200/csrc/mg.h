@@ -52,11 +52,12 @@ struct MgHost {
     std::vector<int32_t> mem_s, mem_c, chunk_mem, row_at;
     std::vector<int2> chunk_fine;
 };
-// Members with fewer rows have no hierarchy and are solved by one block each (jcg_small.cu).  961 rows: 0.37
-// ms alone, 1.46 with the hierarchy; 256 members of 900 rows 0.64 and 3.3 ms.  Beside a 40,000-row member the
-// block's time adds to the solve's (900 rows: 2.7 ms, 2.3 with the hierarchy), and more with every row, so
-// the line stays at the size that a block's threads hold two rows of.
-constexpr int kMgMinRows = 1024;
+// Members with fewer rows have no hierarchy and are solved by one block each (jcg_small.cu).  A solve alone, by
+// one block and with the hierarchy: 961 rows 0.37 and 1.46 ms, 2,025 rows 0.72 and 1.77, 3,969 rows 1.43 and
+// 1.92; on short channels the gap is larger (63 x 20 nodes, 6 steps 3.4 and 14.1 ms).  64 members of 3,969 rows
+// 2.0 and 3.4 ms.  Beside a 40,000-row member the block's time adds to the solve's (2,025 rows: 3.0 ms, 2.3 with the
+// hierarchy).  The line is where a block's threads hold eight rows each; there the two are close.
+constexpr int kMgMinRows = 4096;
 // nnp_s/nnp: node -> nodes of the batch (global rows, ball order); row0/rows per member.
 // A member has a hierarchy from kMgMinRows rows on, unless one of its coarse rows has more neighbours than
 // a map byte can name: a property of the member alone.  Returns false when a matrix needs more than 32-bit

@@ -233,7 +233,8 @@ gs_status gs_get_stats(gs_ctx* ctx, int member, gs_stats* out);
    GS_K_NODAL_VEL and GS_K_NODAL_TRACER take up to 1024 threads and run with 256 at most;
    gs_get_launch reports the shape that runs.
    GS_K_JCG_TILES: a = tiles a large member is cut into, b = the smallest tile in rows (a
-   multiple of 32); this changes the order of the solver's partial sums.  A change takes effect
+   multiple of 32); this changes the order of the solver's partial sums (in GS_FP32_IR not for members below
+   4,096 rows, which have no tiles).  A change takes effect
    at the next launch (the captured step is recaptured). */
 enum {
     GS_K_BTRACK = 0, GS_K_SIDE_PREP = 1, GS_K_GHAT = 2, GS_K_ASSEMBLE = 3, GS_K_MOMENTUM = 4,

@@ -125,9 +125,10 @@ def test_batch_is_no_slower_than_its_members_one_after_another(native):
     assert times[0] <= sum(times[1:]), times
 
 
-@pytest.mark.parametrize("side", [31, 32, 33])
-def test_elevation_at_the_line(native, oracle_lib, side):
-    """Both sides of the 1,024-row line between a block's own solve and the hierarchy, against the oracle."""
+@pytest.mark.parametrize("side", [31, 32, 33, 45, 46, 63, 64])
+def test_elevation_at_the_lines(native, oracle_lib, side):
+    """Both sides of the lines between two, four and eight rows a thread of a block's own solve (1,024 and 2,048
+    rows) and between it and the hierarchy (4,096), against the oracle."""
     from gschism_b200.model import Model
     from oracle.step_api import OracleModel
     c = _basin(50 + side, side)
@@ -145,7 +146,7 @@ def test_small_and_large_members_equal_their_solo_runs(native, inner_maxiter):
     """Members on both sides of the line in one context, bit for bit their solo results; with one or two
     iterations a sweep every member leaves the hierarchy after sweeps that do not halve the residual."""
     from gschism_b200.model import Model
-    cs = [_basin(61, 20), _basin(62, 31), _basin(63, 32), _basin(64, 90)]
+    cs = [_basin(61, 20), _basin(62, 33), _basin(63, 63), _basin(64, 64), _basin(65, 90)]
     mix = Model(cs, precision="fp32_ir", ir_inner_maxiter=inner_maxiter)
     mix.step(2)
     for k, c in enumerate(cs):
@@ -160,8 +161,8 @@ def test_small_and_large_members_equal_their_solo_runs(native, inner_maxiter):
 
 @pytest.mark.parametrize("side", [6, 8, 22, 23])
 def test_elevation_of_a_block_member(native, oracle_lib, side):
-    """Members solved by one block: fewer rows than a warp's two slices, and both sides of one row per
-    thread, against the oracle."""
+    """Small members solved by one block: fewer rows than two slices, and both sides of one row per thread,
+    against the oracle."""
     from gschism_b200.model import Model
     from oracle.step_api import OracleModel
     c = _basin(70 + side, side)
@@ -177,7 +178,7 @@ def test_elevation_of_a_block_member(native, oracle_lib, side):
 def test_parked_block_member_is_done_at_once(native):
     """A zero right-hand side: solved by x = 0 without an iteration, beside members that iterate."""
     from gschism_b200.model import Model
-    cs = [_basin(81, 20), _basin(82, 25), _basin(83, 40)]
+    cs = [_basin(81, 20), _basin(82, 25), _basin(83, 70)]
     m = Model(cs, precision="fp32_ir")
     m.park(0, m.member_state(0))
     m.step(2)
@@ -196,7 +197,7 @@ def test_timed_out_block_member_is_reported_and_the_context_recovers(native):
     a large member: the wait runs out, is reported once, and the context steps on bit for bit."""
     from gschism_b200 import _lib as L
     from gschism_b200.model import Model
-    for cs in ([_basin(84, 20)], [_basin(84, 20), _basin(85, 50)]):
+    for cs in ([_basin(84, 20)], [_basin(84, 20), _basin(85, 70)]):
         ref, m = (Model(cs, precision="fp32_ir") for _ in range(2))
         ref.step(3)
         m.step(2)
@@ -250,3 +251,18 @@ def test_fp64_members_of_shared_blocks_equal_their_solo_runs(native, sides):
         assert mix.stats(k)["jcg_iters"] == solo.stats(0)["jcg_iters"]
         solo.close()
     mix.close()
+
+
+def test_block_member_gets_the_same_bits_in_every_form(native):
+    """A thread of a block's solve holds as many rows as the context's largest small member needs; a member's
+    bits do not depend on that."""
+    from gschism_b200.model import Model
+    small = _basin(91, 24)
+    solo = Model([small], precision="fp32_ir")
+    solo.step(3)
+    for side in (40, 60):
+        m = Model([_basin(92, side), small], precision="fp32_ir")
+        m.step(3)
+        assert np.array_equal(m.get(1, "ETA2"), solo.get(0, "ETA2")), side
+        m.close()
+    solo.close()

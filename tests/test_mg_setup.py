@@ -62,10 +62,10 @@ def _members(mg, graphs):
     return mem_c
 
 
-@pytest.mark.parametrize("nx,ny,on", [(20, 20, False), (31, 33, False), (32, 32, True), (50, 50, True), (63, 63, True)])
+@pytest.mark.parametrize("nx,ny,on", [(20, 20, False), (63, 65, False), (64, 64, True), (80, 90, True)])
 def test_line_between_plain_and_hierarchy(mg, nx, ny, on):
-    """1,023 rows and fewer iterate without the hierarchy, alone and beside a large member."""
-    g, big = _lattice(nx, ny), _lattice(70, 70)
+    """4,095 rows and fewer have no hierarchy, alone and beside a large member."""
+    g, big = _lattice(nx, ny), _lattice(110, 90)
     assert (_members(mg, [g])[0] >= 0) == on
     c = _members(mg, [g, big])
     assert (c[0] >= 0) == on and c[1] >= 0
@@ -84,7 +84,7 @@ def _hub(n, spokes):
 def test_wide_coarse_row_drops_only_its_own_member(mg, spokes, on):
     """A coarse row of more than 255 neighbours leaves that member without the hierarchy; its neighbours in
     the batch keep theirs, as they would alone."""
-    hub, other = _hub(8 * 320, spokes), _lattice(40, 40)
+    hub, other = _hub(8 * 600, spokes), _lattice(70, 70)
     assert (_members(mg, [hub])[0] >= 0) == on
     for batch, k in (([other, hub, other], 1), ([hub, other], 0)):
         c = _members(mg, batch)
@@ -100,7 +100,7 @@ def test_wide_row_on_a_higher_level(mg):
         a, b = k % 16, 16 * (k + 10)
         g[a].append(b)
         g[b].append(a)
-    other = _lattice(40, 40)
+    other = _lattice(70, 70)
     c = _members(mg, [other, g, other])
     assert c[0] >= 0 and c[1] < 0 and c[2] >= 0
 
