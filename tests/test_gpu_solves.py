@@ -192,18 +192,20 @@ def test_parked_block_member_is_done_at_once(native):
     m.close()
 
 
-def test_timed_out_block_member_is_reported_and_the_context_recovers(native):
+def test_timed_out_member_is_reported_and_the_context_recovers(native):
     """The recovery path (test_gpu_recovery.py) with a stalled member that one block solves, alone and beside
-    a large member: the wait runs out, is reported once, and the context steps on bit for bit."""
+    a large member, and with the large one stalled: the wait runs out, is reported once, and the context
+    steps on bit for bit."""
     from gschism_b200 import _lib as L
     from gschism_b200.model import Model
-    for cs in ([_basin(84, 20)], [_basin(84, 20), _basin(85, 70)]):
+    both = [_basin(84, 20), _basin(85, 70)]
+    for cs, stalled in ((both[:1], 0), (both, 0), (both, 1)):
         ref, m = (Model(cs, precision="fp32_ir") for _ in range(2))
         ref.step(3)
         m.step(2)
         saved = [m.member_state(k) for k in range(len(cs))]
         m.set_wait_limit(1 << 14)
-        m.test_stall_solve(0)
+        m.test_stall_solve(stalled)
         m.step(1)
         with pytest.raises(L.GsError) as ei:
             m.sync()
